@@ -274,3 +274,89 @@ def tolerance(case):
     # with its attention in 64 bits differs by 0.021 (largest value 0.24), the streamed blocks with 1 ulp of noise on
     # their modulation vectors by 0.025 (1.2) -- the difference of two equally good quantisations, so it saturates there.
     return {"rel": 3e-2, "max": 0.99}
+
+
+# -- the same results in 64 bits --------------------------------------------------------------
+
+
+def _f16(b):
+    return b.contiguous().view(torch.float16).double()          # [..., 2] bytes -> [..., 1]
+
+
+def _dequant(fmt, w, k):
+    """[n][row bytes] of GGUF blocks -> [n][k] in f64."""
+    if fmt in ("q8_0", "q4_0", "iq4_nl"):
+        b = w.reshape(w.shape[0], k // 32, -1)
+        d = _f16(b[..., :2])
+        if fmt == "q8_0":
+            v = b[..., 2:].contiguous().view(torch.int8).double()
+        else:
+            q = torch.cat([b[..., 2:] & 15, b[..., 2:] >> 4], dim=-1)
+            if fmt == "q4_0":
+                v = q.double() - 8
+            else:
+                table = torch.tensor([-127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113],
+                                     dtype=torch.float64, device=w.device)
+                v = table[q.long()]
+        return (d * v).reshape(-1, k)
+    b = w.reshape(w.shape[0], k // 256, -1)
+    if fmt == "q6_k":
+        ql, qh = b[..., :128].unflatten(-1, (2, 2, 32)), b[..., 128:192].unflatten(-1, (2, 1, 32))
+        low = torch.cat([ql & 15, ql >> 4], dim=-2)                                      # [.., half, 4, 32]
+        high = torch.cat([(qh >> (2 * p)) & 3 for p in range(4)], dim=-2)
+        sc = b[..., 192:208].contiguous().view(torch.int8).double().unsqueeze(-1)
+        q = ((low | (high << 4)).double() - 32).flatten(-3).unflatten(-1, (16, 16))
+        return (_f16(b[..., 208:210]).unsqueeze(-1) * sc * q).reshape(-1, k)
+    d, dmin, s = _f16(b[..., 0:2]), _f16(b[..., 2:4]), b[..., 4:16]
+    sc = torch.cat([s[..., :4] & 63, (s[..., 8:] & 15) | (s[..., :4] >> 6 << 4)], dim=-1)
+    mn = torch.cat([s[..., 4:8] & 63, (s[..., 8:] >> 4) | (s[..., 4:8] >> 6 << 4)], dim=-1)
+    qs = b[..., -128:].unflatten(-1, (4, 1, 32))
+    q = torch.cat([qs & 15, qs >> 4], dim=-2).flatten(-3, -2)                              # [.., 8, 32]
+    if fmt == "q5_k":
+        q = q | torch.stack([(b[..., 16:48] >> i & 1) << 4 for i in range(8)], dim=-2)
+    return ((d * sc.double()).unsqueeze(-1) * q.double() - (dmin * mn.double()).unsqueeze(-1)).reshape(-1, k)
+
+
+def _q8_1(x):
+    """The values that the activation quantiser of the decode linears leaves: 32 of them share one scale."""
+    b = x.unflatten(-1, (-1, 32))
+    amax = b.abs().amax(-1, keepdim=True)
+    q = torch.where(amax > 0, torch.round(b * (127.0 / amax)), torch.zeros_like(b))       # f32: the same ties
+    return ((amax / 127.0).double() * q.double()).flatten(-2)
+
+
+def _gguf_linear(fmt, w, x, k):
+    rows = max(1, (1 << 27) // k)
+    return torch.cat([x @ _dequant(fmt, w[r:r + rows], k).T for r in range(0, w.shape[0], rows)], dim=1)
+
+
+def _rotate(x):
+    """Every 256 columns times the orthonormal Hadamard matrix that is the Kronecker power of the 4 x 4 one."""
+    h4 = torch.tensor([[1, 1, 1, -1], [1, 1, -1, 1], [1, -1, 1, 1], [-1, 1, 1, 1]], dtype=torch.float64, device=x.device)
+    h = torch.kron(torch.kron(h4, h4), torch.kron(h4, h4)) / 16
+    return (x.double().unflatten(-1, (-1, 256)) @ h.T).flatten(-2)
+
+
+def exact(case, seed):
+    """The quantised operands as they are, everything after them in 64 bits.  None for the transformer blocks: their
+    linears quantise what the one before computed, so their results have no value that every correct rounding is near."""
+    kind = case["kind"]
+    if kind == "dit":
+        return None
+    s = prepare(case, seed)
+    if kind == "linear":
+        maxq = 127 if case["bits"] == 8 else 7
+        r = _rotate(s["x"])
+        a = (r.abs().amax(1, keepdim=True) / maxq).clamp_min(1e-12)
+        q = torch.sign(r) * torch.floor((r / a).abs() + 0.5)
+        w = s["w"]
+        if case["bits"] == 4:
+            n = torch.stack([w & 15, w >> 4], dim=-1).flatten(-2)
+            w = n.to(torch.int8) - 16 * (n > 7).to(torch.int8)
+        return (q @ w.double().T) * a * s["w_scale"].double()
+    if kind == "gemv_f32":
+        return _gguf_linear("q8_0", s["w"], s["x"].double(), case["k"])
+    if kind == "gemv":
+        return _gguf_linear(case["fmt"], s["w"], _q8_1(s["x"]), case["k"])
+    of = {"q": "attn_in", "k": "attn_in", "v": "attn_in", "o": "attn_out", "gate": "mlp_in", "up": "mlp_in", "down": "mlp_act"}
+    return [_gguf_linear(fmt, s["w"][name], _q8_1(s["x"][of[name]]), k) for name, fmt, _, k in _layer_shapes(case)]
