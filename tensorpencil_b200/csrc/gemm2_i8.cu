@@ -348,13 +348,6 @@ int launch_pair(tpb_handle_t h, cudaStream_t st, const GemmParams &p, const int8
 
 }  // namespace
 
-// True when the two-CTA kernel should take this problem: enough 256 x 256 tiles to
-// occupy every SM pair.
-bool tpb_gemm2_wants(tpb_handle_t h, int64_t m, int64_t n) {
-    const int64_t tiles = ((m + 255) / 256) * ((n + 255) / 256);
-    return tiles >= h->sm_count / 2;
-}
-
 int tpb_launch_gemm2_silu_pair(tpb_handle_t h, cudaStream_t st, const tpb_gemm::GemmParams &p, int y_dtype,
                                const int8_t *q, const void *w_gate, const void *w_up) {
     if (y_dtype == TPB_F32) return launch_silu_pair<OUT_F32>(h, st, p, q, w_gate, w_up);

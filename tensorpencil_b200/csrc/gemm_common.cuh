@@ -25,10 +25,13 @@ struct TileCfg {
     static constexpr int kStageBytesA = BM * BK;
     static constexpr int kStageBytesB = BN * BK;
     static constexpr int kStageBytes = kStageBytesA + kStageBytesB;
-    static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
-    static constexpr int kTmemCols = 2 * BN;  // two accumulator buffers (power of two >= 32)
-    // epilogue staging: 4 warps x 2 buffers x (32 rows x 128 bytes)
-    static constexpr int kStagingBytes = 4 * 2 * 4096;
+    static constexpr int kStages = BN == 256 ? 4 : BN == 192 ? 5 : BN == 128 ? 6 : 8;
+    static constexpr int kTmemCols = BN == 192 ? 512 : 2 * BN;  // two accumulator buffers (power of two >= 32)
+    // epilogue staging: 4 warps x 2 buffers x (32 rows x 128 bytes); one buffer each at BN = 192, where the second
+    // would cost the fifth operand stage (m 1111, n 3072, k 12288: 38.4 us with four stages, 34.5 with five)
+    static constexpr bool kOneStaging = BN == 192;
+    static constexpr int kStagingPerWarp = kOneStaging ? 4096 : 8192;
+    static constexpr int kStagingBytes = 4 * kStagingPerWarp;
     // tiles + staging + barriers (full/empty per stage, full/empty per accumulator)
     // + TMEM base slot + abort flag, plus 1 KB slack to align the tiles to 1024 bytes.
     static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;

@@ -6,7 +6,7 @@
 // One persistent CTA per SM walks output tiles of 128 x BN:
 //   warp 0      : TMA producer -- 128-byte-swizzled tiles of q and w, K block of
 //                 128 bytes per pipeline stage, completion on an mbarrier;
-//   warp 1      : allocates TMEM and issues tcgen05.mma.kind::i8 (M=128, N=BN,
+//   warp 1      : allocates TMEM and issues tcgen05.mma.kind::i8 (M=128, N=BN = 64 .. 256,
 //                 K=32) from one thread; int32 accumulators live in TMEM, two
 //                 buffers so the epilogue of tile t overlaps the main loop of t+1;
 //   warps 2..5  : epilogue -- tcgen05.ld the accumulator rows (the load of the
@@ -22,7 +22,6 @@
 
 #include "gemm_common.cuh"
 
-bool tpb_gemm2_wants(tpb_handle_t h, int64_t m, int64_t n);
 int tpb_launch_gemm2_group(tpb_handle_t h, cudaStream_t st, const tpb_gemm::GemmParams &p, int y_dtype, const int8_t *q,
                            int count, const void *const *w8, const float *const *w_scale, void *const *y);
 int tpb_launch_gemm2_silu_pair(tpb_handle_t h, cudaStream_t st, const tpb_gemm::GemmParams &p, int y_dtype,
@@ -153,8 +152,8 @@ convrot_gemm_kernel(const __grid_constant__ CUtensorMap tma_a,
     } else {
         // ---------------- epilogue ----------------
         const int quarter = warp & 3;  // TMEM lane quarter this warp may access
-        // two 4 KB staging buffers per warp, each 32 rows x 128 bytes, 1024-byte aligned
-        const uint32_t stg = stg_base + (uint32_t)(warp - 2) * 8192u;
+        // two 4 KB staging buffers per warp (BN = 192: one), each 32 rows x 128 bytes, 1024-byte aligned
+        const uint32_t stg = stg_base + (uint32_t)(warp - 2) * (uint32_t)Cfg::kStagingPerWarp;
         const uint32_t my_row_off = (uint32_t)lane * 128u;
         const uint32_t sw = (uint32_t)(lane & 7);  // 128-byte swizzle: 16-byte piece j of row r sits at j ^ (r & 7)
         uint32_t n_store = 0;                      // stores issued by this warp (selects the staging buffer)
@@ -178,7 +177,7 @@ convrot_gemm_kernel(const __grid_constant__ CUtensorMap tma_a,
             if (p.act_sum != nullptr && row_ok) corr = 8 * __ldcg(p.act_sum + row);
             const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
 
-            epilogue_tile<BN, OUT, PEERS>(t_row, p, &tma_y, stg, my_row_off, sw, n_store, row0, n0, as, corr, lane);
+            epilogue_tile<BN, OUT, PEERS, false, Cfg::kOneStaging>(t_row, p, &tma_y, stg, my_row_off, sw, n_store, row0, n0, as, corr, lane);
             // all of this warp's TMEM reads are complete: hand the buffer back
             tc_fence_before();
             __syncwarp();
@@ -234,20 +233,67 @@ template <int BN, int OUT>
 int launch_cfg(tpb_handle_t h, cudaStream_t st, const GemmParams &p, const int8_t *q, const void *w8,
                bool b_unsigned) {
     if (p.gate != nullptr) return launch_cfg_p<BN, OUT_F32, 3>(h, st, p, q, w8, b_unsigned);
-    if (p.mc_y != nullptr) return launch_cfg_p<BN, OUT, 2>(h, st, p, q, w8, b_unsigned);
-    return p.n_peers > 0 ? launch_cfg_p<BN, OUT, 1>(h, st, p, q, w8, b_unsigned)
-                         : launch_cfg_p<BN, OUT, 0>(h, st, p, q, w8, b_unsigned);
+    if constexpr (BN != 192) {   // pick_tile_peers
+        if (p.mc_y != nullptr) return launch_cfg_p<BN, OUT, 2>(h, st, p, q, w8, b_unsigned);
+        if (p.n_peers > 0) return launch_cfg_p<BN, OUT, 1>(h, st, p, q, w8, b_unsigned);
+    }
+    return launch_cfg_p<BN, OUT, 0>(h, st, p, q, w8, b_unsigned);
+}
+
+// Which tile takes a problem: the one whose waves of tiles cost least.  A persistent CTA (or CTA pair) walks whole
+// tiles, so a launch takes ceil(tiles / SMs) rounds of k / 128 K blocks each, plus what does not overlap (launch,
+// pipeline fill, the last epilogue).  Measured per round and K block of 128 at k = 12288, and the rest at k = 3072 (us):
+//   128 x 64    0.295 + 3.0    (bound by shared-memory traffic: A is staged for 64 columns only)
+//   128 x 128   0.315 + 4.0
+//   128 x 192   0.365 + 4.3
+//   128 x 256   0.46  + 5.0
+//   256 x 256   0.41  + 5.5    on an SM pair
+// (256 x 192 on a pair took 0.39 a round: 0.95 of the 256-wide round for 0.75 of the work, never the best.)  E.g. m 1111,
+// n 3072, k 12288: 216 tiles of 128 x 128 are two rounds, 60 us; 144 of 128 x 192 are one, 34.5 us.  m 777, n 2048, k 4096:
+// two rounds of 128 x 64 28 us, one of 128 x 128 15 us.  m 2048, n 3072, k 12288: 96 pair tiles on 74 pairs 77 us,
+// 256 of 128 x 192 65 us.  The pair keeps a problem unless another tile is 4 % better: under the power cap, which a long
+// GEMM meets, its fewer bytes staged per product count for more than the bursts above show.
+enum Tile { S64, S128, S192, S256, P256 };
+double tile_us(int sms, Tile t, int64_t m, int64_t n, int64_t k, int count) {
+    static const struct { int bm, bn, sms; double per_block, fixed; } kCost[] = {
+        {128, 64, 1, 0.295, 3.0}, {128, 128, 1, 0.315, 4.0}, {128, 192, 1, 0.365, 4.3}, {128, 256, 1, 0.46, 5.0}, {256, 256, 2, 0.41, 5.5}};
+    const auto &c = kCost[t];
+    const int64_t tiles = (m + c.bm - 1) / c.bm * ((n + c.bn - 1) / c.bn) * count;
+    const int64_t slots = sms / c.sms > 0 ? sms / c.sms : 1;
+    return (double)((tiles + slots - 1) / slots) * (double)(k / BK) * c.per_block + c.fixed;
+}
+Tile pick_tile(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double *us = nullptr) {
+    Tile best = S64;
+    double t_best = 0.0;
+    for (int t = S64; t <= P256; t++) {
+        if (t == P256 && h->opt_gemm_one_cta) break;
+        double v = tile_us(h->sm_count, (Tile)t, m, n, k, 1);
+        if (t == P256) v *= 0.96;
+        if (t == S64 || v < t_best) {
+            best = (Tile)t;
+            t_best = v;
+        }
+    }
+    if (us) *us = t_best;
+    return best;
+}
+// The fused all-gather's epilogue also writes every other GPU's copy of the output, which the costs above do not hold:
+// there the widest tile that still gives every SM (pair) work.
+Tile pick_tile_peers(tpb_handle_t h, int64_t m, int64_t n) {
+    auto tiles = [&](int bm, int bn) { return (m + bm - 1) / bm * ((n + bn - 1) / bn); };
+    if (!h->opt_gemm_one_cta && tiles(256, 256) >= h->sm_count / 2) return P256;
+    return tiles(128, 256) >= h->sm_count ? S256 : tiles(128, 128) >= h->sm_count ? S128 : S64;
 }
 
 template <int OUT>
 int launch_out(tpb_handle_t h, cudaStream_t st, const GemmParams &p, const int8_t *q, const void *w8,
-               bool b_unsigned) {
-    // Widest tile that still gives every SM work; narrow tiles for small problems.
-    const int m_tiles = (p.m + BM - 1) / BM;
-    auto tiles = [&](int bn) { return m_tiles * ((p.n + bn - 1) / bn); };
-    if (tiles(256) >= h->sm_count) return launch_cfg<256, OUT>(h, st, p, q, w8, b_unsigned);
-    if (tiles(128) >= h->sm_count) return launch_cfg<128, OUT>(h, st, p, q, w8, b_unsigned);
-    return launch_cfg<64, OUT>(h, st, p, q, w8, b_unsigned);
+               bool b_unsigned, Tile tile) {
+    switch (tile) {
+        case S256: return launch_cfg<256, OUT>(h, st, p, q, w8, b_unsigned);
+        case S192: return launch_cfg<192, OUT>(h, st, p, q, w8, b_unsigned);
+        case S128: return launch_cfg<128, OUT>(h, st, p, q, w8, b_unsigned);
+        default: return launch_cfg<64, OUT>(h, st, p, q, w8, b_unsigned);
+    }
 }
 
 }  // namespace
@@ -283,7 +329,6 @@ int tpb_launch_gemm(tpb_handle_t h, cudaStream_t st, void *y, int y_dtype, int64
     p.k = (int)k;
     p.status = h->d_status;
     const void *w8 = w;
-    const bool one_cta_only = h->opt_gemm_one_cta;
     if (w_bits == 4 && n_peers == 0 && mc_y == nullptr && gate == nullptr && h->opt_w4_fused &&
         ((m + 127) / 128) * ((n + 255) / 256) >= h->sm_count) {
         // opt-in: the packed weight is unpacked inside the GEMM (one-CTA kernel)
@@ -298,13 +343,13 @@ int tpb_launch_gemm(tpb_handle_t h, cudaStream_t st, void *y, int y_dtype, int64
         if (rc != TPB_OK) return rc;
         w8 = buf;
     }
-    // Large problems: two-CTA tiles (256 x 256 per SM pair).  TPB_GEMM_ONE_CTA=1 keeps
-    // the one-CTA kernel for comparisons.
-    if (!one_cta_only && tpb_gemm2_wants(h, m, n)) return tpb_launch_gemm2(h, st, p, y_dtype, q, w8, false);
+    // TPB_GEMM_ONE_CTA=1 keeps the one-CTA kernel for comparisons.
+    const Tile tile = n_peers > 0 || mc_y != nullptr ? pick_tile_peers(h, m, n) : pick_tile(h, m, n, k);
+    if (tile == P256) return tpb_launch_gemm2(h, st, p, y_dtype, q, w8, false);
     switch (y_dtype) {
-        case TPB_F32: return launch_out<OUT_F32>(h, st, p, q, w8, false);
-        case TPB_BF16: return launch_out<OUT_BF16>(h, st, p, q, w8, false);
-        case TPB_S32: return launch_out<OUT_S32>(h, st, p, q, w8, false);
+        case TPB_F32: return launch_out<OUT_F32>(h, st, p, q, w8, false, tile);
+        case TPB_BF16: return launch_out<OUT_BF16>(h, st, p, q, w8, false, tile);
+        case TPB_S32: return launch_out<OUT_S32>(h, st, p, q, w8, false, tile);
     }
     return tpb_fail(h, TPB_ERR_INVALID_ARG, "gemm: unsupported y_dtype %d", y_dtype);
 }
@@ -348,11 +393,15 @@ int tpb_launch_gemm_silu_pair(tpb_handle_t h, cudaStream_t st, void *y, int y_dt
 
 // Up to four weights of one shape times the same activations in one launch of the two-CTA kernel (the q, k, v and
 // gate projections of a DiT block): their tiles follow one another in its persistent loop, so the pipeline fills
-// and drains once instead of once per weight.  Small problems, which the one-CTA kernel takes, run one by one.
+// and drains once instead of once per weight, and the last round is shared by all of them.  One by one where a tile of
+// the one-CTA kernel fits a single weight so much better that it pays (m 256, n = k = 3072: 41 us one by one, 18 together;
+// m 1111, k 12288: 4 x 35 one by one, 141 together).
 int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *const *y, int y_dtype, int64_t ldy,
                           const int8_t *q, const float *act_scale, const void *const *w, const float *const *w_scale,
                           int w_bits, int64_t m, int64_t n, int64_t k) {
-    if (h->opt_gemm_one_cta || !tpb_gemm2_wants(h, m, n)) {
+    double one_us = 0.0;
+    pick_tile(h, m, n, k, &one_us);
+    if (h->opt_gemm_one_cta || 0.96 * tile_us(h->sm_count, P256, m, n, k, count) > count * one_us) {
         for (int g = 0; g < count; g++) {
             const int rc = tpb_launch_gemm(h, st, y[g], y_dtype, ldy, q, act_scale, nullptr, w[g], w_bits, w_scale[g], m, n, k,
                                            nullptr, 0, nullptr, nullptr);

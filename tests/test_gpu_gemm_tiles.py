@@ -1,0 +1,74 @@
+"""The int8 GEMM picks one of five tiles by a cost per round of tiles; these shapes reach each of them (on 148 SMs) with
+row and column counts that are not multiples of the tile, and the group of several weights on both of its routes.  The int32
+accumulators are exact; f32 and bf16 outputs are the two products of the contract, rounded once each."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import oracle  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def be():
+    from tensorpencil_b200.backend import Backend
+    b = Backend(0)
+    yield b
+    b.close()
+
+
+SHAPES = [
+    (130, 1040, 512),      # 128 x 64
+    (777, 2032, 1024),     # 128 x 128
+    (1111, 3056, 512),     # 128 x 192, one round
+    (2000, 3072, 768),     # 128 x 192, two rounds
+    (890, 5360, 1024),     # 128 x 256
+    (2300, 2032, 1024),    # 256 x 256 on an SM pair
+]
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_every_tile_is_exact(be, m, n, k):
+    rng = np.random.default_rng(m + n)
+    q = rng.integers(-127, 128, size=(m, k), dtype=np.int8)
+    w = rng.integers(-128, 128, size=(n, k), dtype=np.int8)
+    s = rng.uniform(0.5, 1.5, m).astype(np.float32)
+    ws = rng.uniform(0.5, 1.5, n).astype(np.float32)
+    acc = oracle.igemm_s32(q, w)
+    f32 = torch.from_numpy((acc.astype(np.float32) * s[:, None]) * ws[None, :])
+    dev = lambda a: torch.from_numpy(a).cuda()
+    be.i8_x, be.i8_scale, be.i8_sum = dev(q.reshape(-1)), dev(s), dev(np.zeros(m, np.int32))
+    be.i8_m, be.i8_cols, be.i8_bits = m, k, 8
+    wd, wsd = dev(w), dev(ws)
+    for dt, want in ((torch.int32, torch.from_numpy(acc)), (torch.float32, f32), (torch.bfloat16, f32.to(torch.bfloat16))):
+        y = torch.full((m, n), 3, dtype=dt, device="cuda")
+        be._gemm(y, wd, wsd, n, 8)
+        be.status_poll()
+        assert torch.equal(y.cpu(), want), dt
+    # the gated residual: x + gate * y, one FMA
+    x = torch.from_numpy(rng.standard_normal((m, n)).astype(np.float32))
+    gate = torch.from_numpy(rng.uniform(-1, 1, n).astype(np.float32))
+    xd = x.cuda()
+    be.gemmGatedAdd(xd, wd, wsd, n, gate.cuda(), 0, 8)
+    be.status_poll()
+    want = x.double() + gate.double() * f32.double()         # the product is exact in f64
+    assert bool(((xd.cpu().double() - want).abs() <= 2.0 ** -24 * want.abs() * (1 + 1e-6) + 1e-45).all())   # one rounding to f32
+
+
+@pytest.mark.parametrize("m,n,k", [(130, 512, 256), (200, 3072, 512), (1111, 768, 2048)])
+def test_group_of_small_weights_matches_the_single_calls(be, m, n, k):
+    rng = np.random.default_rng(7 * m + n)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    be._prep(dev(rng.standard_normal((m, k)).astype(np.float32)), m, k, 8)
+    ws = [dev(rng.integers(-128, 128, size=(n, k), dtype=np.int8)) for _ in range(4)]
+    sc = [dev(rng.uniform(0.5, 1.5, n).astype(np.float32)) for _ in range(4)]
+    for dt in (torch.float32, torch.bfloat16):
+        want = [torch.empty((m, n), dtype=dt, device="cuda") for _ in ws]
+        for y, w, s in zip(want, ws, sc):
+            be._gemm(y, w, s, n, 8)
+        got = [torch.full((m, n), 3.0, dtype=dt, device="cuda") for _ in ws]
+        be.gemmGroup(got, ws, sc, n, 8)
+        be.status_poll()
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), dt
