@@ -314,6 +314,150 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
     }
 }
 
+// The same behind the per-warp rings of q8_0_gemv_q8n_kernel: a warp streams its rows two at a time with bulk copies, a
+// lane takes a block pair of both rows per stage.  f32 activations sit in shared memory, 64 of them every 272 bytes: 16-byte reads
+// at that lane stride fall on distinct banks.  A weight is (32768 + u) * d - 32896 * d in one FMA, u = q + 128 put into
+// the mantissa of 32768 by a byte permute: every step of it is exact (27 bits before, 18 after the FMA's one rounding), so the product
+// q * d is the one the kernel above forms with a conversion and a multiplication.
+//
+// What bounds it: 2.25 instructions a weight for that, the two multiply-adds and their operands from shared memory (16 KB of
+// activations per two rows of 2048), against 62.4 MB of weights at 14336 x 4096 (9.4 us at 6.65 TB/s): 77.8 us with the
+// 16-bit global loads of the kernel above -> 16.0 us = 3.9 TB/s; 17408 x 5120 23 us, 4096 x 14336 13.9 us, 1024 x 4096 2.8 us.
+constexpr int kF32PairBytes = 272;
+__global__ void __launch_bounds__(512, 1)
+q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ w, float scale, int rows, int cols, int stages,
+                          uint32_t *status) {
+    constexpr int R = 2;
+    constexpr int kStageBytes = stage_bytes(R);
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int n_warps = blockDim.x >> 5;
+    const int nblk = cols / 32;
+    const size_t row_bytes = (size_t)nblk * kBlockBytes;
+    uint8_t *ring0 = smem + (size_t)(nblk / 2) * kF32PairBytes;
+    const uint32_t ring = smem_u32(ring0) + (uint32_t)(warp * stages * kStageBytes);
+    const uint32_t bars = smem_u32(ring0) + (uint32_t)(n_warps * stages * kStageBytes) + (uint32_t)(warp * stages * 8);
+
+    if (lane == 0) {
+        for (int s = 0; s < stages; s++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8 * s), "r"(1));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    tpb_grid_dep_launch();
+
+    const int cpr = (nblk + kChunkBlocks - 1) / kChunkBlocks;  // chunks per row
+    const int gw = blockIdx.x * n_warps + warp;
+    const int GW = gridDim.x * n_warps;
+    const int my_r0 = (int)((long long)rows * gw / GW);
+    const int my_r1 = (int)((long long)rows * (gw + 1) / GW);
+    const int total = (my_r1 - my_r0 + R - 1) / R * cpr;
+
+    int is_c = 0, is_row = my_r0, is_st = 0;
+    auto issue = [&]() {   // lane 0: the copies of the next iteration into its stage
+        const int nrow = min(R, my_r1 - is_row);
+        const uint32_t bytes = (uint32_t)min(kChunkBlocks, nblk - is_c * kChunkBlocks) * kBlockBytes;
+        const uint32_t bar = bars + 8 * is_st;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes * (uint32_t)nrow) : "memory");
+        const uint8_t *src = w + (size_t)is_row * row_bytes + (size_t)is_c * kChunkBytes;
+        for (int r = 0; r < nrow; r++)
+            bulk_g2s(ring + (uint32_t)(is_st * kStageBytes + r * kChunkBytes), src + (size_t)r * row_bytes, bytes, bar);
+        if (++is_st == stages) is_st = 0;
+        if (++is_c == cpr) {
+            is_c = 0;
+            is_row += R;
+        }
+    };
+    // weights are constants: they start before the kernel in front has finished
+    if (lane == 0)
+        for (int i = 0; i < stages - 1 && i < total; i++) issue();
+
+    tpb_grid_dep_wait();
+    for (int i = threadIdx.x; i < cols / 4; i += blockDim.x)
+        *reinterpret_cast<float4 *>(smem + (size_t)(i >> 4) * kF32PairBytes + (i & 15) * 16) = __ldcg(reinterpret_cast<const float4 *>(x) + i);
+    __syncthreads();
+
+    f2 acc[R] = {};
+    int st = 0, c = 0, row0 = my_r0;
+    uint32_t par = 0;
+    for (int i = 0; i < total; i++) {
+        if (lane == 0 && i + stages - 1 < total) {   // the stage consumed in iteration i - 1 (warp-synchronous)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue();
+        }
+        const bool ok = mbar_wait(bars + 8 * st, par, status, (13u << 24) | (uint32_t)st);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        const int pair = c * kPairsPerChunk + lane;
+        if (2 * pair < nblk) {      // nblk is even
+            const uint32_t wl = ring + (uint32_t)(st * kStageBytes + lane * 2 * kBlockBytes);
+            const uint8_t *xp = smem + (size_t)pair * kF32PairBytes;
+            // block by block: its eight quant words of both rows, then the 32 activations once
+            uint32_t tw[R][8];
+            f2 d2[R], c2[R];
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    // words 0..8 of the pair hold block 0 (d in the low half of word 0), words 8..16 block 1 (d in
+                    // the high half of word 8); with an odd row count the second row reads a stage's old bytes, unused
+                    const uint32_t a = wl + (uint32_t)(r * kChunkBytes);
+                    float d;
+                    if (half == 0) {
+                        uint32_t prev = lds32(a);
+                        d = f16lo(prev);
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const uint32_t next = lds32(a + 4u * (j + 1));
+                            tw[r][j] = __funnelshift_r(prev, next, 16) ^ 0x80808080u;
+                            prev = next;
+                        }
+                    } else {
+                        d = f16hi(lds32(a + 32u));
+#pragma unroll
+                        for (int j = 0; j < 8; j++) tw[r][j] = lds32(a + 36u + 4u * j) ^ 0x80808080u;
+                    }
+                    d2[r] = pack2(d, d);
+                    c2[r] = pack2(-32896.0f * d, -32896.0f * d);
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const ulonglong2 xv = *reinterpret_cast<const ulonglong2 *>(xp + half * 128 + j * 16);
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const uint32_t q = tw[r][j];
+                        const f2 w01 = fma2(pack2i((int)__byte_perm(q, 0x47000000u, 0x7404), (int)__byte_perm(q, 0x47000000u, 0x7414)), d2[r], c2[r]);
+                        const f2 w23 = fma2(pack2i((int)__byte_perm(q, 0x47000000u, 0x7424), (int)__byte_perm(q, 0x47000000u, 0x7434)), d2[r], c2[r]);
+                        acc[r] = fma2(w01, xv.x, acc[r]);
+                        acc[r] = fma2(w23, xv.y, acc[r]);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (c == cpr - 1) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[r]));
+                float v = lo + hi;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0 && row0 + r < my_r1) y[row0 + r] = v * scale;
+                acc[r] = 0ull;
+            }
+            c = 0;
+            row0 += R;
+        } else {
+            c++;
+        }
+        if (++st == stages) {
+            st = 0;
+            par ^= 1u;
+        }
+    }
+}
+
 // Launch with programmatic stream serialisation: the kernel may begin before the
 // previous kernel in the stream has finished; it orders itself with griddepcontrol.wait.
 template <typename Kern>
@@ -520,6 +664,23 @@ int tpb_launch_q8_0_gemv_f32(tpb_handle_t h, cudaStream_t st, float *y, const fl
     const size_t smem = (size_t)cols * 4;
     if (smem > (size_t)h->smem_optin)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "q8_0_gemv_f32: cols too large for shared memory");
+    // Rows of whole 16-byte words (what a bulk copy can start at): the ring kernel, the faster one from the smallest decode
+    // shape on (1024 x 4096 2.8 us), with as many warps and stages as fit beside the activations (to some 40000 columns)
+    if (cols % 256 == 0) {
+        const size_t act = (size_t)(cols / 64) * kF32PairBytes;
+        int warps = 0, stages = 0;
+        dp4a_plan(h, act, rows, stage_bytes(2), 16, &warps, &stages);
+        if (warps != 0) {
+            int rgrid = (int)((rows + 2 * warps - 1) / (2 * warps));
+            if (rgrid > h->sm_count) rgrid = h->sm_count;
+            static tpb_per_device_once ring_set;
+            TPB_CUDA(h, tpb_set_max_smem_once(h, q8_0_gemv_f32_ring_kernel, h->smem_optin, ring_set));
+            TPB_CUDA(h, tpb_launch_pdl(q8_0_gemv_f32_ring_kernel, dim3((unsigned)rgrid), dim3((unsigned)(warps * 32)),
+                                       act + (size_t)warps * stages * (stage_bytes(2) + 8) + 64, st, y, x,
+                                       reinterpret_cast<const uint8_t *>(w), scale, (int)rows, (int)cols, stages, h->d_status));
+            return TPB_OK;
+        }
+    }
     static tpb_per_device_once smem_set;
     TPB_CUDA(h, tpb_set_max_smem_once(h, q8_0_gemv_f32_kernel, h->smem_optin, smem_set));
     int grid = (int)((rows + 7) / 8);

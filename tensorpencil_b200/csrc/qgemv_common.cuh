@@ -1,6 +1,9 @@
-// Pieces shared by the decode GEMV kernels (qgemv.cu, qgemv_k.cu): the bounded mbarrier wait
-// and the 1-D bulk copy that feed their per-warp shared-memory rings.
+// Pieces shared by the decode GEMV kernels (qgemv.cu, qgemv_mma.cu, qgemv_k.cu, qgemv_kmma.cu): the bounded
+// mbarrier wait and the 1-D bulk copy that feed their shared-memory rings, packed f32 arithmetic and the field
+// decoders of the GGUF formats.
 #pragma once
+
+#include <cuda_fp16.h>
 
 #include "tpb_internal.h"
 
@@ -50,5 +53,92 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
         "l"(src), "r"(bytes), "r"(bar)
         : "memory");
 }
+
+
+// Two packed f32 values; each half rounds like the scalar instruction.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+    f2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ f2 pack2i(int lo, int hi) {
+    f2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+    return d;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+    f2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// Shared-memory loads by 32-bit shared address: one address register instead of a generic pointer pair.
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ float f16lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xffffu))); }
+__device__ __forceinline__ float f16hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
+
+
+enum { FMT_Q4_0 = 1, FMT_Q4_K = 2, FMT_Q5_K = 3, FMT_Q6_K = 4, FMT_IQ4_NL = 5 };
+
+// Four 4-bit indices (one per byte of idx, 0..15) -> the four signed bytes of ggml's
+// kvalues_iq4nl table: two byte-permutes over the table halves, merged by the index's bit 3.
+__device__ __forceinline__ uint32_t iq4nl_lookup(uint32_t idx) {
+    constexpr uint32_t T0 = 0xBFAD9881u;  // -127 -104 -83 -65
+    constexpr uint32_t T1 = 0xF6EADDCFu;  // -49 -35 -22 -10
+    constexpr uint32_t T2 = 0x26190D01u;  // 1 13 25 38
+    constexpr uint32_t T3 = 0x71594535u;  // 53 69 89 113
+    const uint32_t t = idx & 0x07070707u;
+    const uint32_t u = t | (t >> 4);                     // byte 0: b0 | b1 << 4, byte 2: b2 | b3 << 4
+    const uint32_t sel = __byte_perm(u, 0, 0x4420);      // 16-bit selector b0, b1, b2, b3
+    const uint32_t v_lo = __byte_perm(T0, T1, sel);
+    const uint32_t v_hi = __byte_perm(T2, T3, sel);
+    const uint32_t m = ((idx >> 3) & 0x01010101u) * 0xffu;
+    return (v_lo & ~m) | (v_hi & m);
+}
+
+// The 6-bit scales and mins of sub-blocks 2j and 2j+1 (j = 0..3) of a q4_k / q5_k super-block, both pairs at
+// once and without a branch; s0, s1, s2 are the three words of the 12-byte scales field.  ggml's
+// get_scale_min_k4 read two sub-blocks at a time: bytes 2j, 2j+1 of the field are one 16-bit word, and
+//   j < 2:  scale = byte & 63 of word j of s0,              min = byte & 63 of word j of s1
+//   j >= 2: scale = (s2 word & 0x0f0f) | (s0 word >> 6 << 4), min = (s2 word >> 4 & 0x0f0f) | (s1 word >> 6 << 4)
+// with "word" the 16-bit half number (j & 1) of each 32-bit word.
+__device__ __forceinline__ void scale_min_k4_pair(int j, uint32_t s0, uint32_t s1, uint32_t s2, float &sc0, float &mn0,
+                                                  float &sc1, float &mn1) {
+    const uint32_t sh = (uint32_t)(j & 1) * 16u;
+    const uint32_t a = (s0 >> sh) & 0xffffu, b = (s1 >> sh) & 0xffffu, c = (s2 >> sh) & 0xffffu;
+    const bool upper = j >= 2;
+    const uint32_t s16 = upper ? ((c & 0x0f0fu) | ((a & 0xc0c0u) >> 2)) : (a & 0x3f3fu);
+    const uint32_t m16 = upper ? (((c >> 4) & 0x0f0fu) | ((b & 0xc0c0u) >> 2)) : (b & 0x3f3fu);
+    sc0 = (float)(s16 & 0xffu);
+    sc1 = (float)(s16 >> 8);
+    mn0 = (float)(m16 & 0xffu);
+    mn1 = (float)(m16 >> 8);
+}
+
 
 }  // namespace tpb_gemv

@@ -32,8 +32,6 @@ using namespace tpb_gemv;
 
 namespace {
 
-enum { FMT_Q4_0 = 1, FMT_Q4_K = 2, FMT_Q5_K = 3, FMT_IQ4_NL = 5 };
-
 // A lane takes U 64-element units per pipeline stage (template parameter: 2, or 3 where that saves iterations
 // per row -- K = 5120 is 80 units: two chunks of 64, the second a quarter full, or one chunk of 96).
 constexpr int kActPairBytes = 80;   // a unit's 64 activation bytes + 16 pad (bank-conflict-free 16-byte reads)
@@ -63,43 +61,6 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
     asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
-// Four 4-bit indices (one per byte of idx, 0..15) -> the four signed bytes of ggml's
-// kvalues_iq4nl table: two byte-permutes over the table halves, merged by the index's bit 3.
-__device__ __forceinline__ uint32_t iq4nl_lookup(uint32_t idx) {
-    constexpr uint32_t T0 = 0xBFAD9881u;  // -127 -104 -83 -65
-    constexpr uint32_t T1 = 0xF6EADDCFu;  // -49 -35 -22 -10
-    constexpr uint32_t T2 = 0x26190D01u;  // 1 13 25 38
-    constexpr uint32_t T3 = 0x71594535u;  // 53 69 89 113
-    const uint32_t t = idx & 0x07070707u;
-    const uint32_t u = t | (t >> 4);                     // byte 0: b0 | b1 << 4, byte 2: b2 | b3 << 4
-    const uint32_t sel = __byte_perm(u, 0, 0x4420);      // 16-bit selector b0, b1, b2, b3
-    const uint32_t v_lo = __byte_perm(T0, T1, sel);
-    const uint32_t v_hi = __byte_perm(T2, T3, sel);
-    const uint32_t m = ((idx >> 3) & 0x01010101u) * 0xffu;
-    return (v_lo & ~m) | (v_hi & m);
-}
-__device__ __forceinline__ float f16lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xffffu))); }
-__device__ __forceinline__ float f16hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
-
-// The 6-bit scales and mins of sub-blocks 2j and 2j+1 (j = 0..3) of a q4_k / q5_k super-block, both pairs at
-// once and without a branch; s0, s1, s2 are the three words of the 12-byte scales field.  ggml's
-// get_scale_min_k4 read two sub-blocks at a time: bytes 2j, 2j+1 of the field are one 16-bit word, and
-//   j < 2:  scale = byte & 63 of word j of s0,              min = byte & 63 of word j of s1
-//   j >= 2: scale = (s2 word & 0x0f0f) | (s0 word >> 6 << 4), min = (s2 word >> 4 & 0x0f0f) | (s1 word >> 6 << 4)
-// with "word" the 16-bit half number (j & 1) of each 32-bit word.
-__device__ __forceinline__ void scale_min_k4_pair(int j, uint32_t s0, uint32_t s1, uint32_t s2, float &sc0, float &mn0,
-                                                  float &sc1, float &mn1) {
-    const uint32_t sh = (uint32_t)(j & 1) * 16u;
-    const uint32_t a = (s0 >> sh) & 0xffffu, b = (s1 >> sh) & 0xffffu, c = (s2 >> sh) & 0xffffu;
-    const bool upper = j >= 2;
-    const uint32_t s16 = upper ? ((c & 0x0f0fu) | ((a & 0xc0c0u) >> 2)) : (a & 0x3f3fu);
-    const uint32_t m16 = upper ? (((c >> 4) & 0x0f0fu) | ((b & 0xc0c0u) >> 2)) : (b & 0x3f3fu);
-    sc0 = (float)(s16 & 0xffu);
-    sc1 = (float)(s16 >> 8);
-    mn0 = (float)(m16 & 0xffu);
-    mn1 = (float)(m16 >> 8);
-}
-
 // The arithmetic of one pipeline stage: rows 0 .. nrow - 1 of `stage` (pitch bytes apart) hold chunk c of their
 // weight rows; every lane decodes its U units of each row and adds their dot products with the M activation
 // rows into acc.

@@ -156,3 +156,18 @@ def test_q6k_weight_at_the_very_end_of_its_allocation(be):
     be.opGemvQuantQ8N("q6_k", y, store[off:off + nbytes], 1.0, n, k, 3, 0, 3)
     be.status_poll()
     assert np.array_equal(y.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n,k", [(1, 256), (7, 768), (33, 2304), (300, 4096), (2500, 1024), (149, 17408), (20, 32768), (9, 96)])
+def test_q8_0_gemv_f32_at_the_edges_of_its_rings(be, n, k):
+    """The single-row GEMV on f32 activations: one row, odd rows per warp, rows of less than a chunk, a chunk and a bit, many chunks,
+    the activations that leave the fewest rings, and a row length that bulk copies cannot take (the plain kernel)."""
+    w = synth.gguf_weights("q8_0", n, k, seed=n + k)
+    x = np.random.default_rng(n).standard_normal(k).astype(np.float32)
+    y = torch.full((n,), float("nan"), dtype=torch.float32, device="cuda")
+    be.opGemvQuant("q8_0", y, torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), 0.5, n, k)
+    be.status_poll()
+    wf = np.stack([oracle.q8_0_dequant_row(w[r], k) for r in range(n)]).astype(np.float64)
+    err = np.abs(y.cpu().numpy() - 0.5 * (wf @ x.astype(np.float64)))
+    # a lane adds at most 64 products per 2048 columns, then six steps to the row's sum, each with an error of at most 2^-24 of sum |w||x|
+    assert (err <= 0.5 * (64 * -(-k // 2048) + 6) * 2.0 ** -24 * (np.abs(wf) @ np.abs(x.astype(np.float64))) + 1e-9).all()
