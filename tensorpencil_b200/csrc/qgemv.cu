@@ -266,12 +266,13 @@ q8_0_gemv_q8n_simple_kernel(const GemvParams p) {
 // q8_1 activation quantiser: one warp per 32-element block
 // (src/gpu/cuda/elt.zig:1226-1269).
 __global__ void __launch_bounds__(256)
-q8_1_quantize_kernel(const float *__restrict__ x, float *__restrict__ d, int8_t *__restrict__ qs,
-                     int nblk) {
+q8_1_quantize_kernel(const float *x, float *d, int8_t *qs, int nblk) {
+    tpb_grid_dep_launch();   // the GEMV behind this starts on its weights, which no kernel writes
+    tpb_grid_dep_wait();
     const int blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (blk >= nblk) return;
-    const float xi = x[(size_t)blk * 32 + lane];
+    const float xi = __ldcg(x + (size_t)blk * 32 + lane);
     float amax = fabsf(xi);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -582,8 +583,10 @@ int tpb_launch_q8_1_quantize(tpb_handle_t h, cudaStream_t st, const float *x, in
     int8_t *qs = reinterpret_cast<int8_t *>(xq) + (size_t)nblk * 4;
     const int block = 256;
     const int grid = (nblk * 32 + block - 1) / block;
-    q8_1_quantize_kernel<<<grid, block, 0, st>>>(x, d, qs, nblk);
-    TPB_CUDA(h, cudaGetLastError());
+    // A programmatic dependent launch, like every kernel of the decode path.  As a plain launch it waited for the GEMV in front to
+    // leave the GPU, and the one behind could not fill its rings meanwhile: quantiser + GEMV of 1024 x 4096 5.5 -> 4.2 us, of
+    // 17408 x 5120 20.2 -> 18.1 us, the eleven launches of an 8B model's layer 61.8 -> 53.8 us (GPU time, one token).
+    TPB_CUDA(h, tpb_launch_pdl(q8_1_quantize_kernel, dim3((unsigned)grid), dim3(block), 0, st, x, d, qs, nblk));
     return TPB_OK;
 }
 
