@@ -6,10 +6,13 @@ fallback implementation behind these functions.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libtpb200.so")
+CALL_PATH = os.path.join(_HERE, "lib", "_tpbcall.so")
 
 TPB_OK = 0
 TPB_ERR_INVALID_ARG = -1
@@ -107,3 +110,21 @@ def load() -> C.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_calls = None
+
+
+def load_calls():
+    """The same functions, for the calls made once per weight, without ctypes' argument conversion (csrc/pycall.c):
+    pointers and integers as Python integers (None = NULL), scales as floats."""
+    global _calls
+    if _calls is None:
+        load()
+        if not os.path.exists(CALL_PATH):
+            raise RuntimeError(f"{CALL_PATH} is missing: build it with `python -m tensorpencil_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_tpbcall", CALL_PATH)
+        spec = importlib.util.spec_from_loader("_tpbcall", loader)
+        _calls = importlib.util.module_from_spec(spec)
+        loader.exec_module(_calls)
+    return _calls

@@ -28,7 +28,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import TPB_BF16, TPB_F16, TPB_F32, TPB_OK, TPB_S32, TpbError
+from ._lib import GGUF_FMT, TPB_BF16, TPB_F16, TPB_F32, TPB_OK, TPB_S32, TpbError
 
 _TORCH_TO_TPB = {torch.float32: TPB_F32, torch.bfloat16: TPB_BF16, torch.float16: TPB_F16,
                  torch.int32: TPB_S32}
@@ -54,6 +54,10 @@ class Backend:
         if rc != TPB_OK:
             raise TpbError(rc, self.lib.tpb_status_string(rc).decode())
         self.h = h
+        # for the calls made once per weight: native argument passing, and the raw handle and device index it takes
+        self._calls = _lib.load_calls()
+        self._hv = h.value
+        self._index = device
         # prep -> GEMM state (backend.zig:336-341)
         self.i8_x: Optional[torch.Tensor] = None
         self.i8_scale: Optional[torch.Tensor] = None
@@ -74,6 +78,7 @@ class Backend:
             torch.cuda.synchronize(self.device)
             self.lib.tpb_destroy(self.h)
             self.h = None
+            self._hv = None
 
     def __del__(self):
         try:
@@ -82,7 +87,8 @@ class Backend:
             pass
 
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream
+        # the raw handle, without the torch.cuda.Stream object around it (1.5 us a call)
+        return torch._C._cuda_getCurrentRawStream(self._index)
 
     def _check(self, rc: int):
         if rc != TPB_OK:
@@ -152,7 +158,7 @@ class Backend:
         if self.i8_scale is None or self.i8_scale.numel() < m:
             self.i8_scale = torch.empty(max(m, 1), dtype=torch.float32, device=self.device)
             self.i8_sum = torch.empty(max(m, 1), dtype=torch.int32, device=self.device)
-        rc = self.lib.tpb_convrot_prep(self.h, self._stream(), x.data_ptr(), _TORCH_TO_TPB[x.dtype],
+        rc = self._calls.tpb_convrot_prep(self._hv, self._stream(), x.data_ptr(), _TORCH_TO_TPB[x.dtype],
                                        m, cols, bits, self.i8_x.data_ptr(),
                                        self.i8_scale.data_ptr(), self.i8_sum.data_ptr())
         self._check(rc)
@@ -296,7 +302,7 @@ class Backend:
         ydt = _TORCH_TO_TPB[y.dtype]
         if w_bits == 4:
             self.reserveW4(rows, self.i8_cols)
-        rc = self.lib.tpb_convrot_gemm(self.h, self._stream(), y.data_ptr(), ydt,
+        rc = self._calls.tpb_convrot_gemm(self._hv, self._stream(), y.data_ptr(), ydt,
                                        ldy if ldy is not None else rows,
                                        self.i8_x.data_ptr(), self.i8_scale.data_ptr(),
                                        self.i8_sum.data_ptr() if w_bits == 4 else None,
@@ -372,26 +378,30 @@ class Backend:
         """Quantise f32 activations (cols = total element count, a multiple of
         32) into the shared q8 scratch: f32 d[cols/32] then int8 qs[cols]
         (backend.zig:1687-1695)."""
+        xq = self._q8_scratch(x, cols)
+        rc = self._calls.tpb_q8_1_quantize(self._hv, self._stream(), x.data_ptr(), cols, xq.data_ptr())
+        self._check(rc)
+        self.launches += 1
+
+    def _q8_scratch(self, x: torch.Tensor, cols: int) -> torch.Tensor:
         assert x.dtype == torch.float32 and x.is_cuda and cols % 32 == 0
         need = cols // 32 * 4 + cols
         if self.q8_act is None or self.q8_act.numel() < need:
             self.q8_act = torch.empty(need, dtype=torch.uint8, device=self.device)
         self._q8_total = cols
-        rc = self.lib.tpb_q8_1_quantize(self.h, self._stream(), x.data_ptr(), cols, self.q8_act.data_ptr())
-        self._check(rc)
-        self.launches += 1
+        return self.q8_act
 
     def opGemvQuantQ8N(self, dt: str, y: torch.Tensor, w_bytes, scale: float, rows: int, cols: int,
                        ng: int, row_off: int, n_total: int):
         """Grouped dp4a GEMV: y[i][rows] = scale * (W @ x_hat[row_off+i]) for i < ng <= 8
         against the activations staged by ONE opGemvQuantizeX(x, n_total*cols)
         (backend.zig:1719-1735)."""
-        from ._lib import GGUF_FMT
-        if dt not in GGUF_FMT:
+        fmt = GGUF_FMT.get(dt)
+        if fmt is None:
             raise NotImplementedError(f"GEMV weight format {dt!r} is not implemented (q8_0, q4_0, q4_k, q5_k, q6_k, iq4_nl are)")
         assert self.q8_act is not None and self._q8_total == n_total * cols
         w_dev = self.cachedWeight(w_bytes) if isinstance(w_bytes, np.ndarray) else w_bytes
-        rc = self.lib.tpb_gguf_gemv_q8n(self.h, self._stream(), GGUF_FMT[dt], y.data_ptr(), w_dev.data_ptr(),
+        rc = self._calls.tpb_gguf_gemv_q8n(self._hv, self._stream(), fmt, y.data_ptr(), w_dev.data_ptr(),
                                         float(scale), rows, cols, self.q8_act.data_ptr(), ng,
                                         row_off, n_total)
         self._check(rc)
@@ -403,7 +413,7 @@ class Backend:
         if dt != "q8_0":
             raise NotImplementedError(f"GEMV weight format {dt!r} is outside this library's scope")
         w_dev = self.cachedWeight(w_bytes) if isinstance(w_bytes, np.ndarray) else w_bytes
-        rc = self.lib.tpb_q8_0_gemv_f32(self.h, self._stream(), y.data_ptr(), x.data_ptr(),
+        rc = self._calls.tpb_q8_0_gemv_f32(self._hv, self._stream(), y.data_ptr(), x.data_ptr(),
                                         w_dev.data_ptr(), float(scale), rows, cols)
         self._check(rc)
         self.launches += 1
@@ -428,7 +438,7 @@ class Backend:
             self.i8_sum = torch.empty(max(m, 1), dtype=torch.int32, device=self.device)
         if bits == 4:
             self.reserveW4(n, k)
-        rc = self.lib.tpb_convrot_linear(self.h, self._stream(), y.data_ptr(), _TORCH_TO_TPB[y.dtype], n,
+        rc = self._calls.tpb_convrot_linear(self._hv, self._stream(), y.data_ptr(), _TORCH_TO_TPB[y.dtype], n,
                                          x.data_ptr(), _TORCH_TO_TPB[x.dtype], self.i8_x.data_ptr(),
                                          self.i8_scale.data_ptr(), self.i8_sum.data_ptr(), w.data_ptr(), bits,
                                          _ptr(w_scale), m, n, k)
@@ -485,7 +495,7 @@ class Backend:
             cur.wait_event(ev)
             if not copy_only:
                 self._prep(self._host_x[r0:r1], r1 - r0, k, bits)
-                rc = self.lib.tpb_convrot_gemm(self.h, self._stream(), self._host_y[r0:r1].data_ptr(), ydt, n,
+                rc = self._calls.tpb_convrot_gemm(self._hv, self._stream(), self._host_y[r0:r1].data_ptr(), ydt, n,
                                                self.i8_x.data_ptr(), self.i8_scale.data_ptr(), None,
                                                w8.data_ptr(), 8, _ptr(w_scale), r1 - r0, n, k)
                 self._check(rc)
@@ -503,8 +513,10 @@ class Backend:
         grouped GEMV per 8 activation rows."""
         m = x.shape[0]
         y = torch.empty((m, n), dtype=torch.float32, device=self.device)
-        self.opGemvQuantizeX(x, m * k)
-        for r0 in range(0, m, 8):
-            ng = min(8, m - r0)
-            self.opGemvQuantQ8N("q8_0", y[r0:], w, scale, n, k, ng, r0, m)
+        xq = self._q8_scratch(x, m * k)
+        w_dev = self.cachedWeight(w) if isinstance(w, np.ndarray) else w
+        # opGemvQuantizeX, then opGemvQuantQ8N per group, without returning to Python in between
+        self._check(self._calls.q8_0_linear(self._hv, self._stream(), y.data_ptr(), x.data_ptr(), m, w_dev.data_ptr(),
+                                            float(scale), n, k, xq.data_ptr()))
+        self.launches += 1 + (m + 7) // 8
         return y

@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -20,6 +21,7 @@ CSRC = os.path.join(PKG, "csrc")
 OUT_DIR = os.path.join(PKG, "lib")
 LIB = os.path.join(OUT_DIR, "libtpb200.so")
 OBJ_DIR = os.path.join(OUT_DIR, "obj")
+PYCALL = os.path.join(OUT_DIR, "_tpbcall.so")   # CPython entry to the hot calls (csrc/pycall.c)
 
 SOURCES = ["api.cu", "prep.cu", "prep_fused.cu", "gemm_i8.cu", "gemm2_i8.cu", "gemm_w4.cu", "qgemv.cu", "qgemv_mma.cu", "qgemv_k.cu", "offload.cu", "peer.cu", "attn.cu"]
 
@@ -75,6 +77,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-cudart", "static",
                                                      "-Xlinker", "--no-undefined"]
         subprocess.run(cmd, check=True, env=env)
+    src = os.path.join(CSRC, "pycall.c")
+    if force or _stale(PYCALL, [src, headers[0]]):
+        subprocess.run(["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"],
+                        "-I", os.path.join(ROOT, "include"), src, "-o", PYCALL, "-L", OUT_DIR, "-l:libtpb200.so",
+                        "-Wl,-rpath,$ORIGIN"], check=True)
     return LIB
 
 
