@@ -89,6 +89,7 @@ constexpr int kMaxWarpsWide = 16;
 #endif
 constexpr bool kF32LoadFirst = TPB_F32_LOAD_FIRST != 0;   // rows of the gated preps: one unit per half-warp, more warps per row
 constexpr int kTilePairs = 16 * 18;  // 64-bit slots of one half-warp's tile (2304 bytes)
+constexpr size_t kMaxPrepSmem = (size_t)kMaxWarpsWide * 2 * kTilePairs * 8;   // of the widest row's CTA
 
 // Two packed f32 values; every operation rounds each half like the scalar instruction.
 typedef unsigned long long f2;
@@ -520,9 +521,11 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
         const size_t smem = ACT_ONLY ? 0 : (size_t)kRowsPerCta * 2 * kTilePairs * sizeof(f2);
         err = tpb_launch_pdl(convrot_prep_kernel<T, 1, OP, ACT_ONLY, true>, grid, block, smem, st, P);
     } else {
-        // The gated preps do more arithmetic per element and gain from more warps per row (one unit per
-        // half-warp, up to 16 warps) while the row still fits that way; the plain prep does not.
-        const bool wide = (OP == OP_SILU_MUL || OP == OP_SIGMOID_MUL) && n_units <= 2 * kMaxWarpsWide;
+        // One unit per half-warp, up to 16 warps a row, while the row fits that way (k <= 16384): the warps a row has in flight
+        // hide its latencies, and with two units each they were half as many.  Against 8 warps of two units (us, bf16): SiLU gate
+        // 4608 x 12288 152 -> 82, RMS norm 104 -> 98, 1111 x 9216 21.6 -> 19.5, plain 1111 x 9216 14.1 -> 13.2, 512 x 12288 11.3 -> 10.1,
+        // 4608 x 12288 58.1 -> 57.9.
+        const bool wide = n_units <= 2 * kMaxWarpsWide;
         const int max_warps = wide ? kMaxWarpsWide : kMaxWarps;
         const int upw = (n_units + 2 * max_warps - 1) / (2 * max_warps);  // 1..4 for k <= 32768
         const int warps = (n_units + 2 * upw - 1) / (2 * upw);
@@ -531,7 +534,8 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
 #define TPB_PREP_CASE(UU)                                                                               \
     case UU: {                                                                                          \
         auto kern = convrot_prep_kernel<T, UU, OP, ACT_ONLY, false>;                                    \
-        if (smem > 48 * 1024) err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        static tpb_per_device_once smem_set;                                                            \
+        if (smem > 48 * 1024) err = tpb_set_max_smem_once(h, kern, (int)kMaxPrepSmem, smem_set);        \
         if (err == cudaSuccess) err = tpb_launch_pdl(kern, grid, block, smem, st, P);                   \
         break;                                                                                          \
     }
