@@ -5,7 +5,8 @@
 // multicast); q8_1 activations (int8 + per-32-block scale) stay in shared memory for the
 // kernel's life; dp4a for the integer dots, f32 accumulation, warp butterfly, * scale.
 // A second kernel with the same arithmetic behind one CTA-wide ring (kquant_gemv_ring_kernel,
-// further down) takes the calls with one or two activation rows whose rows are long or many.
+// further down) takes the calls with one or two activation rows whose rows are long or many, and a third on mma.sync
+// (qgemv_kmma.cu) those with several activation rows of large weights; all three give the same bits.
 //
 // The unit of work of a lane is 64 consecutive elements (two q8_1 activation blocks):
 //   q4_0  a pair of 18-byte blocks (f16 d + 16 nibble bytes each; 36 bytes = 9 aligned
@@ -29,6 +30,10 @@
 #include "qgemv_common.cuh"
 
 using namespace tpb_gemv;
+
+bool tpb_kquant_mma_fits(tpb_handle_t h, int fmt, int64_t rows, int64_t cols);
+int tpb_launch_kquant_mma(tpb_handle_t h, cudaStream_t st, int fmt, float *y, const uint8_t *w, float scale, int64_t rows,
+                          int64_t cols, const float *xd, const int8_t *xq, int m);
 
 namespace {
 
@@ -835,11 +840,28 @@ q6k_gemv_ring_kernel(const KGemvParams p, const int stages) {
     }
 }
 
-// TPB_GEMVK_KERNEL=ring|warp forces one of the two kernels (read at every launch, for measurements).
+// TPB_GEMVK_KERNEL=ring|warp|mma forces one of the kernels where it takes the call (read at every launch, for measurements).
 static int k_kernel_override() {
     const char *e = getenv("TPB_GEMVK_KERNEL");
     if (e == nullptr) return 0;
-    return e[0] == 'r' ? 1 : e[0] == 'w' ? 2 : 0;
+    return e[0] == 'r' ? 1 : e[0] == 'w' ? 2 : e[0] == 'm' ? 3 : 0;
+}
+
+// Whether the mma.sync kernel (qgemv_kmma.cu: the same bits, nearly the same time for any number of activation rows) beats the
+// dp4a kernels, whose time grows by 10-20 % with every row and, on long rows, jumps where the activations crowd the rings out or
+// the group has to be split.  Measured on ten shapes and five formats; us, dp4a / mma, q4_k unless said:
+//   M = 8   1024 x 4096 6.1 / 6.5 (q4_0)   1024 x 5120 8.2 / 7.2   4096 x 4096 8.5 / 8.0   14336 x 4096 22.2 / 15.0
+//   M = 5   4096 x 4096 6.8 / 7.7   9216 x 2304 9.6 / 9.3   2048 x 8192 9.6 / 8.0   5120 x 5120 13.5 / 10.1   17408 x 5120 24.0 / 17.6
+//   M = 4   4096 x 4096 6.2 / 7.6   9216 x 2304 8.6 / 9.2   2048 x 8192 8.4 / 7.7   5120 x 5120 10.6 / 9.9   14336 x 4096 15.2 / 14.5
+//           17408 x 5120 19.1 / 17.5 (q6_k 31.3 / 28.5)   5120 x 17408 26.4 / 26.0 (q5_k 30.4 / 28.2, q6_k 41.4 / 40.4)
+//   M = 3   17408 x 5120 16.9 / 17.7   32000 x 4096 30.0 / 22.8 (q6_k 34.4 / 33.9)
+static bool mma_wins(int64_t rows, int64_t cols, int m) {
+    const int64_t weights = rows * cols;
+    if (m >= 4 && cols >= 8192) return weights >= 16000000;
+    if (m == 8) return weights >= (cols >= 5120 ? 5000000 : 8000000);
+    if (m >= 5) return weights >= 20000000;
+    if (m == 4) return cols >= 4096 && weights >= 25000000;
+    return m == 3 && cols >= 4096 && weights >= 120000000;
 }
 
 template <int M>
@@ -1083,6 +1105,12 @@ int tpb_gguf_gemv_q8n(tpb_handle_t h, tpb_stream_t stream, int fmt, float *y, co
                   "gguf_gemv: need 1 <= ng <= 8 and row_off + ng <= n_total");
     TPB_CHECK_ARG(h, tpb_aligned16(w) && tpb_aligned16(xq), "gguf_gemv: w and xq must be 16-byte aligned");
     if (rows == 0) return TPB_OK;
+    const int nblk = (int)(cols / 32);
+    const int force = k_kernel_override();
+    if ((force == 3 || (force == 0 && mma_wins(rows, cols, ng))) && tpb_kquant_mma_fits(h, fmt, rows, cols))
+        return tpb_launch_kquant_mma(h, (cudaStream_t)stream, fmt, y, reinterpret_cast<const uint8_t *>(w), scale, rows, cols,
+                                     reinterpret_cast<const float *>(xq) + (size_t)row_off * nblk,
+                                     reinterpret_cast<const int8_t *>(xq) + (size_t)n_total * nblk * 4 + (size_t)row_off * cols, ng);
     if (ng > 1 && !kq_group_fits(h, fmt, ng, cols)) {
         // the group's activations would leave no room for the weight rings (eight rows of 17408 columns are
         // 209 KB): two launches with half the activation rows each -- a row's result does not depend on its group
@@ -1093,7 +1121,6 @@ int tpb_gguf_gemv_q8n(tpb_handle_t h, tpb_stream_t stream, int fmt, float *y, co
                                  row_off + first, n_total);
     }
     KGemvParams p;
-    const int nblk = (int)(cols / 32);
     p.y = y;
     p.w = reinterpret_cast<const uint8_t *>(w);
     p.xd = reinterpret_cast<const float *>(xq) + (size_t)row_off * nblk;

@@ -171,3 +171,33 @@ def test_q8_0_gemv_f32_at_the_edges_of_its_rings(be, n, k):
     err = np.abs(y.cpu().numpy() - 0.5 * (wf @ x.astype(np.float64)))
     # a lane adds at most 64 products per 2048 columns, then six steps to the row's sum, each with an error of at most 2^-24 of sum |w||x|
     assert (err <= 0.5 * (64 * -(-k // 2048) + 6) * 2.0 ** -24 * (np.abs(wf) @ np.abs(x.astype(np.float64))) + 1e-9).all()
+
+
+@pytest.mark.parametrize("fmt", ["q4_0", "iq4_nl", "q4_k", "q5_k", "q6_k"])
+@pytest.mark.parametrize("m", [1, 3, 8])
+@pytest.mark.parametrize("n,k", [(1, 256), (17, 768), (33, 4096), (300, 1024), (64, 6144), (165, 9216), (37, 9472), (600, 17408), (18, 26624)])
+def test_gguf_gemv_mma_kernel_gives_the_dp4a_kernels_bits(be, fmt, m, n, k, monkeypatch):
+    """The mma.sync kernel adds the same terms in the same order as the dp4a kernels, so forcing either gives identical bits: one
+    row, rows that leave a 16-row stage partly filled, fewer units than warps, four, five and six units per warp and ones that not
+    all warps have, two and more passes over K with an odd and an even number of groups, a partial last group."""
+    w = synth.gguf_weights(fmt, n, k, seed=3 * n + k)
+    x = (np.random.default_rng(m + n).standard_normal((m, k))).astype(np.float32)
+    monkeypatch.setenv("TPB_GEMVK_KERNEL", "mma")
+    got = run(be, fmt, w, n, k, x)
+    monkeypatch.setenv("TPB_GEMVK_KERNEL", "warp")
+    assert np.array_equal(got, run(be, fmt, w, n, k, x))
+    want = oracle.gguf_gemv_q8(fmt, w, n, k, x)
+    err = np.abs(got.astype(np.float64) - want)
+    assert (err <= 2e-5 * bound(fmt, w, n, k, x) + 1e-6).all(), f"max err {err.max():.3e}"
+
+
+@pytest.mark.parametrize("m", [3, 4, 5, 8])
+@pytest.mark.parametrize("fmt,n,k", [("q4_k", 5100, 5120), ("q5_k", 2050, 8192), ("q6_k", 1030, 17408), ("iq4_nl", 9001, 2304)])
+def test_gguf_gemv_large_weights_give_the_same_bits_on_every_kernel(be, fmt, n, k, m, monkeypatch):
+    """Shapes on both sides of the dispatch rule; many row groups per CTA."""
+    w = synth.gguf_weights(fmt, n, k, seed=n)
+    x = (np.random.default_rng(m).standard_normal((m, k))).astype(np.float32)
+    auto = run(be, fmt, w, n, k, x)
+    for kern in ("mma", "warp"):
+        monkeypatch.setenv("TPB_GEMVK_KERNEL", kern)
+        assert np.array_equal(auto, run(be, fmt, w, n, k, x)), kern
