@@ -291,7 +291,7 @@ class Backend:
                                            self._attn_qb.data_ptr(), self._attn_kb.data_ptr(), self._attn_vt.data_ptr(),
                                            seq, seq, heads, kv_heads, head_dim,
                                            float(scale if scale is not None else head_dim ** -0.5)))
-        self.launches += 4
+        self.launches += 2
         return out
 
     def _gemm(self, y: torch.Tensor, w_bytes: np.ndarray, weight_scale: np.ndarray, rows: int,

@@ -469,52 +469,71 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
     return *reinterpret_cast<const uint32_t *>(&b);
 }
 
-// q [seq][heads*128] and k [seq][kv_heads*128] in one launch: a half-warp per (token, head) of q or
-// of k, a lane holds 8 consecutive elements (four rotation pairs).
+// q [seq][heads*128] and k [seq][kv_heads*128]: a half-warp per two consecutive heads of a token (its q heads first, then its k
+// heads), a lane holds 8 consecutive elements (four rotation pairs) of each.
 //   out [heads][seq][128] bf16 = rope(x * inv_rms(x) * w)
+// Two heads share the lane's cos / sin values (with one head the tables are twice a bf16 row's bytes through L1) and have their
+// loads in flight together; with four, registers cost more resident warps than that gains (seq 4608 x 24 heads bf16: see
+// attn_prepare_kernel).
+constexpr int kHeadsPerUnit = 2;
 template <typename T>
-__global__ void __launch_bounds__(256)
-qk_norm_rope_kernel(const T *__restrict__ q, const T *__restrict__ k, const float *__restrict__ qw,
-                    const float *__restrict__ kw, const float *__restrict__ cosv, const float *__restrict__ sinv,
-                    float eps, int seq, int heads, int kv_heads, __nv_bfloat16 *__restrict__ qb,
-                    __nv_bfloat16 *__restrict__ kb) {
-    tpb_grid_dep_launch();
-    tpb_grid_dep_wait();
+__device__ __forceinline__ void
+qk_norm_rope(const unsigned block, const T *q, const T *k, const float *__restrict__ qw, const float *__restrict__ kw,
+             const float *__restrict__ cosv, const float *__restrict__ sinv, float eps, int seq, int heads, int kv_heads,
+             __nv_bfloat16 *qb, __nv_bfloat16 *kb) {
     const int slots = heads + kv_heads;
-    const long long unit = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    const unsigned groups = (unsigned)(slots + kHeadsPerUnit - 1) / kHeadsPerUnit;   // units per token
+    const unsigned unit = block * 16u + (threadIdx.x >> 4);     // 256 threads = 16 half-warps
     const int l = threadIdx.x & 15;
-    // a whole half-warp leaves together: the shuffles below stay inside it
-    const bool live = unit < (long long)seq * slots;
-    const int p = live ? (int)(unit / slots) : 0;
-    const int sl = live ? (int)(unit - (long long)p * slots) : 0;
-    const bool is_q = sl < heads;
-    const int h = is_q ? sl : sl - heads;
-    const int nh = is_q ? heads : kv_heads;
-    const T *src = (is_q ? q : k) + ((size_t)p * nh + h) * kHd + 8 * l;
-    float v[8];
-    load8(src, v);
-    float ss = 0.0f;
+    const int p = (int)(unit / groups);
+    const int s0 = (int)(unit - (unsigned)p * groups) * kHeadsPerUnit;
+    // a whole half-warp has the same token and heads: the shuffles below stay inside it
+    float v[kHeadsPerUnit][8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) ss += v[i] * v[i];
+    for (int i = 0; i < kHeadsPerUnit; i++) {
+        const int sl = s0 + i;
+        if (p < seq && sl < slots) {
+            const bool is_q = sl < heads;
+            load8((is_q ? q + ((size_t)p * heads + sl) * kHd : k + ((size_t)p * kv_heads + (sl - heads)) * kHd) + 8 * l, v[i]);
+        } else {
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (!live) return;
-    const float inv = __frsqrt_rn(ss * (1.0f / kHd) + eps);
-    const float *w = (is_q ? qw : kw) + 8 * l;
-    const float4 w0 = __ldg(reinterpret_cast<const float4 *>(w)), w1 = __ldg(reinterpret_cast<const float4 *>(w) + 1);
-    const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-    // rotation pairs 4l .. 4l+3 of this position's table
-    const float4 c4 = __ldg(reinterpret_cast<const float4 *>(cosv + (size_t)p * (kHd / 2)) + l);
-    const float4 s4 = __ldg(reinterpret_cast<const float4 *>(sinv + (size_t)p * (kHd / 2)) + l);
-    const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
-    uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float a = v[2 * i] * inv * wv[2 * i], b = v[2 * i + 1] * inv * wv[2 * i + 1];
-        o[i] = bf16_pair(a * cs[i] - b * sn[i], a * sn[i] + b * cs[i]);
+            for (int e = 0; e < 8; e++) v[i][e] = 0.0f;
+        }
     }
-    __nv_bfloat16 *dst = (is_q ? qb : kb) + ((size_t)h * seq + p) * kHd + 8 * l;
-    *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    float cs[4] = {}, sn[4] = {}, wv[8] = {};
+    if (p < seq) {
+        // rotation pairs 4l .. 4l+3 of this position's table
+        const float4 c4 = __ldg(reinterpret_cast<const float4 *>(cosv + (size_t)p * (kHd / 2)) + l);
+        const float4 s4 = __ldg(reinterpret_cast<const float4 *>(sinv + (size_t)p * (kHd / 2)) + l);
+        cs[0] = c4.x; cs[1] = c4.y; cs[2] = c4.z; cs[3] = c4.w;
+        sn[0] = s4.x; sn[1] = s4.y; sn[2] = s4.z; sn[3] = s4.w;
+    }
+#pragma unroll
+    for (int i = 0; i < kHeadsPerUnit; i++) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 8; e++) ss += v[i][e] * v[i][e];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const int sl = s0 + i;
+        if (p >= seq || sl >= slots) continue;
+        const bool is_q = sl < heads;
+        if (i == 0 || sl == heads) {     // this unit's first head, or its first k head
+            const float *w = (is_q ? qw : kw) + 8 * l;
+            const float4 w0 = __ldg(reinterpret_cast<const float4 *>(w)), w1 = __ldg(reinterpret_cast<const float4 *>(w) + 1);
+            wv[0] = w0.x; wv[1] = w0.y; wv[2] = w0.z; wv[3] = w0.w;
+            wv[4] = w1.x; wv[5] = w1.y; wv[6] = w1.z; wv[7] = w1.w;
+        }
+        const float inv = __frsqrt_rn(ss * (1.0f / kHd) + eps);
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float a = v[i][2 * e] * inv * wv[2 * e], b = v[i][2 * e + 1] * inv * wv[2 * e + 1];
+            o[e] = bf16_pair(a * cs[e] - b * sn[e], a * sn[e] + b * cs[e]);
+        }
+        __nv_bfloat16 *dst = (is_q ? qb + ((size_t)sl * seq + p) * kHd : kb + ((size_t)(sl - heads) * seq + p) * kHd) + 8 * l;
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
 }
 
 // v [seq][kv_heads*128] -> vt [kv_heads][128][seq_pad] bf16 (kv contiguous; columns seq..seq_pad-1 zero).
@@ -523,12 +542,9 @@ qk_norm_rope_kernel(const T *__restrict__ q, const T *__restrict__ k, const floa
 // c = c' ^ (d >> 3): a half-warp (same token pair, 16 dim groups) then hits 16 different banks, and
 // the second half-warp works 16 token pairs further on, in the other 16 banks.
 template <typename T>
-__global__ void __launch_bounds__(256)
-v_transpose_kernel(const T *__restrict__ v, int seq, int seq_pad, int kv_heads, __nv_bfloat16 *__restrict__ vt) {
-    __shared__ uint32_t tile[kHd][32];
-    tpb_grid_dep_launch();
-    tpb_grid_dep_wait();
-    const int p0 = blockIdx.x * 64, h = blockIdx.y;
+__device__ __forceinline__ void v_transpose(const unsigned block_tok, const int h, const T *v, int seq, int seq_pad, int kv_heads,
+                                            __nv_bfloat16 *vt, uint32_t (&tile)[kHd][32]) {
+    const int p0 = (int)block_tok * 64;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = lane & 15;                                   // dim group: dims 8c .. 8c+7
 #pragma unroll
@@ -564,6 +580,23 @@ v_transpose_kernel(const T *__restrict__ v, int seq, int seq_pad, int kv_heads, 
             *reinterpret_cast<uint4 *>(vt + ((size_t)h * kHd + d) * seq_pad + t0) =
                 make_uint4(g[0 ^ x], g[1 ^ x], g[2 ^ x], g[3 ^ x]);
     }
+}
+
+// Both in one launch, the transpose's CTAs first: the two are independent, and the second launch's start-up and the last CTAs of
+// the first left HBM idle.  Bound by HBM at large sequences (170 MB at 4608 x 24 bf16, 25.5 us at 6.65 TB/s) and by the launch at small ones.
+// us, two launches with one head per half-warp / one launch with one, two, four heads: seq 4608 x 24 heads bf16 39.8 / 38.5, 36.9, 41.1;
+// 2345 x 24 f32 26.4 / 26.7, 21.9, 23.4; 1024 x 24 bf16 9.7 / 8.8, 7.3, 7.7; 513 x 12 bf16 6.2 / 5.2, 3.7, 4.4.
+template <typename T>
+__global__ void __launch_bounds__(256)
+attn_prepare_kernel(const T *q, const T *k, const T *v, const float *__restrict__ qw, const float *__restrict__ kw,
+                    const float *__restrict__ cosv, const float *__restrict__ sinv, float eps, int seq, int seq_pad, int heads,
+                    int kv_heads, __nv_bfloat16 *qb, __nv_bfloat16 *kb, __nv_bfloat16 *vt, unsigned tok_blocks) {
+    __shared__ uint32_t tile[kHd][32];
+    tpb_grid_dep_launch();
+    tpb_grid_dep_wait();
+    const unsigned n_v = tok_blocks * (unsigned)kv_heads;
+    if (blockIdx.x < n_v) v_transpose<T>(blockIdx.x % tok_blocks, (int)(blockIdx.x / tok_blocks), v, seq, seq_pad, kv_heads, vt, tile);
+    else qk_norm_rope<T>(blockIdx.x - n_v, q, k, qw, kw, cosv, sinv, eps, seq, heads, kv_heads, qb, kb);
 }
 
 // 2-D bf16 tensor [rows][cols] (cols contiguous), box = 64 columns x 128 rows, 128-byte swizzle,
@@ -607,20 +640,16 @@ int tpb_attn_prepare(tpb_handle_t h, tpb_stream_t stream, const void *q, const v
     cudaStream_t st = (cudaStream_t)stream;
     const int seq_pad = (int)((seq + 7) / 8 * 8);
     const dim3 blk(256);
-    const long long units = (long long)seq * (heads + kv_heads);     // half-warps
-    const dim3 gqk((unsigned)((units + 15) / 16));
-    const dim3 gv((unsigned)((seq_pad + 63) / 64), (unsigned)kv_heads);
-    cudaError_t e;
-    if (in_dtype == TPB_F32) {
-        e = tpb_launch_pdl(qk_norm_rope_kernel<float>, gqk, blk, 0, st, (const float *)q, (const float *)k, q_norm, k_norm,
-                           cosv, sinv, eps, (int)seq, heads, kv_heads, (__nv_bfloat16 *)qb, (__nv_bfloat16 *)kb);
-        if (e == cudaSuccess) e = tpb_launch_pdl(v_transpose_kernel<float>, gv, blk, 0, st, (const float *)v, (int)seq, seq_pad, kv_heads, (__nv_bfloat16 *)vt);
-    } else {
-        e = tpb_launch_pdl(qk_norm_rope_kernel<__nv_bfloat16>, gqk, blk, 0, st, (const __nv_bfloat16 *)q,
-                           (const __nv_bfloat16 *)k, q_norm, k_norm, cosv, sinv, eps, (int)seq, heads, kv_heads,
-                           (__nv_bfloat16 *)qb, (__nv_bfloat16 *)kb);
-        if (e == cudaSuccess) e = tpb_launch_pdl(v_transpose_kernel<__nv_bfloat16>, gv, blk, 0, st, (const __nv_bfloat16 *)v, (int)seq, seq_pad, kv_heads, (__nv_bfloat16 *)vt);
-    }
+    const long long units = (long long)seq * ((heads + kv_heads + kHeadsPerUnit - 1) / kHeadsPerUnit);     // half-warps
+    const unsigned tok_blocks = (unsigned)((seq_pad + 63) / 64);
+    const dim3 grid((unsigned)((units + 15) / 16) + tok_blocks * (unsigned)kv_heads);     // < 2^28 by the check above
+    const auto launch = [&](auto *tag) {
+        using T = std::remove_pointer_t<decltype(tag)>;
+        return tpb_launch_pdl(attn_prepare_kernel<T>, grid, blk, 0, st, (const T *)q, (const T *)k, (const T *)v, q_norm, k_norm, cosv, sinv,
+                              eps, (int)seq, seq_pad, heads, kv_heads, (__nv_bfloat16 *)qb, (__nv_bfloat16 *)kb, (__nv_bfloat16 *)vt,
+                              tok_blocks);
+    };
+    const cudaError_t e = in_dtype == TPB_F32 ? launch((float *)nullptr) : launch((__nv_bfloat16 *)nullptr);
     TPB_CUDA(h, e);
     return TPB_OK;
 }
