@@ -401,7 +401,10 @@ int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *cons
                           int w_bits, int64_t m, int64_t n, int64_t k) {
     double one_us = 0.0;
     pick_tile(h, m, n, k, &one_us);
-    if (h->opt_gemm_one_cta || 0.96 * tile_us(h->sm_count, P256, m, n, k, count) > count * one_us) {
+    // A reservation that covers one int4 weight only is enough for small problems, as it was when they always ran one by one.
+    const bool small = (m + 255) / 256 * ((n + 255) / 256) < h->sm_count / 2;
+    const bool scratch_for_one = w_bits == 4 && small && h->w4_scratch_bytes < (size_t)count * (size_t)n * (size_t)k;
+    if (h->opt_gemm_one_cta || scratch_for_one || 0.96 * tile_us(h->sm_count, P256, m, n, k, count) > count * one_us) {
         for (int g = 0; g < count; g++) {
             const int rc = tpb_launch_gemm(h, st, y[g], y_dtype, ldy, q, act_scale, nullptr, w[g], w_bits, w_scale[g], m, n, k,
                                            nullptr, 0, nullptr, nullptr);

@@ -72,3 +72,32 @@ def test_group_of_small_weights_matches_the_single_calls(be, m, n, k):
         be.gemmGroup(got, ws, sc, n, 8)
         be.status_poll()
         assert all(torch.equal(a, b) for a, b in zip(got, want)), dt
+
+
+def test_group_of_small_int4_weights_needs_scratch_for_one_only():
+    """Small groups used to run one by one, so a reservation for a single weight served them: it still does (larger groups need
+    all their weights reserved, as the header says)."""
+    from tensorpencil_b200 import _lib
+    from tensorpencil_b200.backend import Backend
+    m, n, k = 200, 512, 512
+    b = Backend(0)
+    rng = np.random.default_rng(3)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    ws = [dev(rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)) for _ in range(3)]
+    sc = [dev(rng.uniform(0.5, 1.5, n).astype(np.float32)) for _ in range(3)]
+    b.reserveW4(n, k)
+    b._w4_reserved = 1 << 40          # the mirror asks for no more
+    b._prep(dev(rng.standard_normal((m, k)).astype(np.float32)), m, k, 4)
+    one = [torch.empty((m, n), dtype=torch.float32, device="cuda") for _ in ws]
+    for y, w, s in zip(one, ws, sc):
+        b._gemm(y, w, s, n, 4)
+    got = [torch.zeros((m, n), dtype=torch.float32, device="cuda") for _ in ws]
+    b.gemmGroup(got, ws, sc, n, 4)
+    b.status_poll()
+    assert all(torch.equal(a, c) for a, c in zip(one, got))
+    wide = [dev(rng.integers(0, 256, size=(4608, k // 2), dtype=np.uint8)) for _ in range(2)]
+    ws2 = [dev(rng.uniform(0.5, 1.5, 4608).astype(np.float32)) for _ in range(2)]
+    b._prep(dev(rng.standard_normal((4096, k)).astype(np.float32)), 4096, k, 4)
+    with pytest.raises(_lib.TpbError):
+        b.gemmGroup([torch.zeros((4096, 4608), device="cuda") for _ in range(2)], wide, ws2, 4608, 4)
+    b.close()
