@@ -323,7 +323,7 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
 //
 // What bounds it: 2.25 instructions a weight for that, the two multiply-adds and their operands from shared memory (16 KB of
 // activations per two rows of 2048), against 62.4 MB of weights at 14336 x 4096 (9.4 us at 6.65 TB/s): 77.8 us with the
-// 16-bit global loads of the kernel above -> 16.0 us = 3.9 TB/s; 17408 x 5120 23 us, 4096 x 14336 13.9 us, 1024 x 4096 2.8 us.
+// 16-bit global loads of the kernel above -> 14.7 us = 4.2 TB/s; 17408 x 5120 21.4 us, 4096 x 14336 13.2 us, 1024 x 4096 2.8 us.
 constexpr int kF32PairBytes = 272;
 __global__ void __launch_bounds__(512, 1)
 q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ w, float scale, int rows, int cols, int stages,
@@ -484,14 +484,14 @@ static GemvOverride gemv_override() {
 // carries ceil(rows / warps_total) rows.  Among the counts that fit (with >= 2 stages and the activations in
 // shared memory) take the one with the best balance; ties go to more warps.  E.g. 5120 rows on 148 SMs:
 // 16 warps -> 2.16 rows per warp (3 vs 2, 72 %), 12 warps -> 2.88 (96 %).
-static void dp4a_plan(tpb_handle_t h, size_t act, int64_t rows, int stage, int max_warps, int *warps, int *stages) {
+static void dp4a_plan(tpb_handle_t h, size_t act, int64_t rows, int stage, int max_warps, int max_stages, int *warps, int *stages) {
     const size_t limit = (size_t)h->smem_optin - 1024;
     *warps = 0;
     *stages = 0;
     double best_eff = -1.0;
     for (int w = max_warps; w >= max_warps / 2; w--) {
         int s_fit = 0;
-        for (int s = 4; s >= 2; s--)
+        for (int s = max_stages; s >= 2; s--)
             if (act + (size_t)w * s * stage + (size_t)w * s * 8 + 64 <= limit) {
                 s_fit = s;
                 break;
@@ -505,6 +505,16 @@ static void dp4a_plan(tpb_handle_t h, size_t act, int64_t rows, int stage, int m
             *stages = s_fit;
         }
     }
+}
+
+// Ring depth of the dp4a kernel.  A warp's copies are issued by its first lane between two steps of arithmetic, and where a warp has few
+// steps the copies of a third and fourth stage delay them more than they save: us at M = 1, 2, 4 with up to four stages / with two:
+// 4096 x 4096 5.3 5.7 7.0 / 4.7 5.2 6.3, 5120 x 5120 8.5 9.5 11.3 / 8.1 8.8 10.9, 11008 x 4096 9.8 10.5 13.3 / 9.6 10.0 12.6, 4096 x 11008
+// 10.1 11.1 13.0 / 9.8 10.6 13.0.  Not for short rows (9216 x 2304 7.3 / 7.5), small weights (1024 x 5120 3.6 / 4.4) or many
+// steps (14336 x 4096 11.7 / 12.2, 8192 x 8192 12.2 / 12.6).
+static int q8n_stages(int64_t rows, int64_t cols) {
+    const double bytes = (double)rows * (double)(cols / 32) * kBlockBytes;
+    return cols >= 4096 && bytes >= 16e6 && bytes < 56e6 ? 2 : 4;
 }
 
 template <int M, int R>
@@ -526,7 +536,7 @@ int launch_q8n_cfg(tpb_handle_t h, cudaStream_t st, const GemvParams &p, int max
         TPB_CUDA(h, launch_pdl(kern, grid, ov.warps * 32, need, st, p, ov.stages));
         return TPB_OK;
     }
-    dp4a_plan(h, act, p.rows, kStage, max_warps, &warps, &stages);
+    dp4a_plan(h, act, p.rows, kStage, max_warps, q8n_stages(p.rows, p.cols), &warps, &stages);
     if (stages == 0) {
         if (R == 2) return TPB_ERR_STATE;
         act_smem = false;
@@ -614,7 +624,7 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
             // the dp4a kernel at its best: fourteen warps with two two-row stages each fit beside the activations
             // (with fewer its time jumps: K = 14336 from the sixth activation row on, K = 28672 from the third)
             int warps = 0, stages = 0;
-            dp4a_plan(h, act_bytes, rows, stage_bytes(2), 16, &warps, &stages);
+            dp4a_plan(h, act_bytes, rows, stage_bytes(2), 16, q8n_stages(rows, cols), &warps, &stages);
             const bool roomy = warps != 0 && act_bytes + 14 * 2 * (size_t)stage_bytes(2) + 14 * 2 * 8 + 64 <=
                                                  (size_t)h->smem_optin - 1024;
             // share of its row slots that hold a row: rows come to a warp two at a time
@@ -672,7 +682,10 @@ int tpb_launch_q8_0_gemv_f32(tpb_handle_t h, cudaStream_t st, float *y, const fl
     if (cols % 256 == 0) {
         const size_t act = (size_t)(cols / 64) * kF32PairBytes;
         int warps = 0, stages = 0;
-        dp4a_plan(h, act, rows, stage_bytes(2), 16, &warps, &stages);
+        // two stages from 16 MB on: 4096 x 4096 6.2 -> 5.5 us, 5120 x 5120 10.7 -> 9.9, 14336 x 4096 15.4 -> 14.7, 32000 x 4096
+        // 25.3 -> 24.2; below, deeper rings bring most of the weight in at once: 1024 x 4096 2.8 us against 3.6, 3072 x 3072 4.7 / 5.8
+        const int max_stages = (double)rows * (double)(cols / 32) * kBlockBytes >= 16e6 ? 2 : 4;
+        dp4a_plan(h, act, rows, stage_bytes(2), 16, max_stages, &warps, &stages);
         if (warps != 0) {
             int rgrid = (int)((rows + 2 * warps - 1) / (2 * warps));
             if (rgrid > h->sm_count) rgrid = h->sm_count;
