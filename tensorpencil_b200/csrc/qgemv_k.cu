@@ -948,11 +948,16 @@ int launch_fmt_mu(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     const size_t act = (size_t)M * (p.cols / 64) * kActPairBytes + (size_t)M * p.nblk * 8;
     // Warps per CTA: every warp owns a contiguous range of whole rows; among the counts that
     // fit with >= 2 stages take the one whose ranges divide most evenly (ties: more warps).
+    // Two stages per ring from 14 MB on: a warp's copies are issued by its first lane between two steps of arithmetic, and those of a
+    // third and fourth stage delay the few steps there are.  us at M = 1, 2, 4, up to four stages / two: q4_k 14336 x 4096 10.6 12.0
+    // 15.2 / 9.8 11.3 14.7, 5120 x 5120 7.8 8.6 10.6 / 7.3 8.2 10.3; q5_k 5120 x 5120 8.6 9.8 12.2 / 8.2 9.2 11.7.  Below, deeper rings bring more
+    // of a small weight in at once (q4_k 2048 x 8192 5.5 / 5.7 at M = 1).
+    const int max_stages = (double)p.rows * (double)p.row_bytes >= 14e6 ? 2 : 4;
     int warps = 0, stages = 0;
     double best_eff = -1.0;
     for (int w = 16; w >= 4; w--) {
         int s_fit = 0;
-        for (int s = 4; s >= 2; s--)
+        for (int s = max_stages; s >= 2; s--)
             if (act + (size_t)w * s * kStage + (size_t)w * s * 8 + 64 <= limit) {
                 s_fit = s;
                 break;
