@@ -264,11 +264,12 @@ q8_0_gemv_q8n_simple_kernel(const GemvParams p) {
 }
 
 // q8_1 activation quantiser: one warp per 32-element block
-// (src/gpu/cuda/elt.zig:1226-1269).
+// (src/gpu/cuda/elt.zig:1226-1269).  Unlike the other kernels it lets its dependent start only once its own wait is over: the
+// GEMV behind it streams its weight before it waits, and a host may have written that weight with the kernel in front of this one.
 __global__ void __launch_bounds__(256)
 q8_1_quantize_kernel(const float *x, float *d, int8_t *qs, int nblk) {
-    tpb_grid_dep_launch();   // the GEMV behind this starts on its weights, which no kernel writes
     tpb_grid_dep_wait();
+    tpb_grid_dep_launch();
     const int blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (blk >= nblk) return;
@@ -593,9 +594,10 @@ int tpb_launch_q8_1_quantize(tpb_handle_t h, cudaStream_t st, const float *x, in
     int8_t *qs = reinterpret_cast<int8_t *>(xq) + (size_t)nblk * 4;
     const int block = 256;
     const int grid = (nblk * 32 + block - 1) / block;
-    // A programmatic dependent launch, like every kernel of the decode path.  As a plain launch it waited for the GEMV in front to
-    // leave the GPU, and the one behind could not fill its rings meanwhile: quantiser + GEMV of 1024 x 4096 5.5 -> 4.2 us, of
-    // 17408 x 5120 20.2 -> 18.1 us, the eleven launches of an 8B model's layer 61.8 -> 53.8 us (GPU time, one token).
+    // A programmatic dependent launch: it starts while the kernel in front drains, and the GEMV behind it fills its rings while it
+    // quantises.  Against a plain launch, GPU time at one token: quantiser + GEMV of 1024 x 4096 5.6 -> 4.6 us, of 17408 x 5120
+    // 20.7 -> 19.7 us, the eleven launches of an 8B model's layer 60.3 -> 55.3 us.  (Letting the GEMV start ahead of the quantiser's wait
+    // gave 4.2, 18.1 and 53.8, but then a weight written in front of the quantiser could be read unfinished.)
     TPB_CUDA(h, tpb_launch_pdl(q8_1_quantize_kernel, dim3((unsigned)grid), dim3(block), 0, st, x, d, qs, nblk));
     return TPB_OK;
 }

@@ -64,3 +64,51 @@ def test_linear_sees_the_activations_of_its_own_iteration(be, bits):
         torch.cuda.synchronize()
     be.status_poll()
     assert all(torch.equal(y, ref[i % 3]) for i, y in enumerate(ys))
+
+
+class _WrittenWeights:
+    """Q8_0 weights whose bytes a kernel writes on the stream just before they are used.  All bytes lie in 0x20 .. 0x2f: as pairs they
+    are finite f16 scales, as quants 32 .. 47, and as words normal f32 numbers, so x = 0 + 1 * source writes them exactly."""
+
+    def __init__(self, be, n, k):
+        self.be, self.n, self.k = be, n, k
+        self.bytes = n * (k // 32) * 34
+        g = torch.Generator(device="cuda").manual_seed(n + k)
+        self.src = [torch.randint(lo, lo + 8, (self.bytes,), dtype=torch.uint8, device="cuda", generator=g).view(torch.float32)
+                    for lo in (0x20, 0x28)]
+        self.w = torch.empty(self.bytes, dtype=torch.uint8, device="cuda")
+        self.one = torch.ones(self.bytes // 4, device="cuda")
+
+    def write(self, i, by):
+        """As the last kernel on the stream: of this library (it lets its successor start early) or of torch."""
+        f = self.w.view(torch.float32)
+        if by == "library":
+            f.zero_()
+            self.be.gatedAdd(f, self.src[i], self.one[:self.bytes // 4], self.bytes // 4, self.bytes // 4, 0)
+        else:
+            torch.add(self.src[i], 0.0, out=f)
+
+
+@pytest.mark.parametrize("by", ["library", "torch"])
+@pytest.mark.parametrize("n,k,m", [(4096, 4096, 1), (17408, 5120, 1), (5120, 17408, 8), (1024, 2048, 4)])
+def test_a_weight_written_before_the_quantiser_is_seen_by_the_gemv(be, n, k, m, by):
+    """write w, quantise x, GEMV: the GEMV reads w early, but not before the kernel in front of the quantiser has finished."""
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        ww = _WrittenWeights(be, n, k)
+        x = torch.randn(m, k, device="cuda")
+        ref = []
+        for i in range(2):
+            ww.write(i, by)
+            torch.cuda.synchronize()
+            assert torch.equal(ww.w.view(torch.int32), ww.src[i].view(torch.int32))
+            ref.append(be.q8_0_linear(x, ww.w, n, k))
+            torch.cuda.synchronize()
+        ys = []
+        for i in range(40):
+            ww.write(i % 2, by)
+            ys.append(be.q8_0_linear(x, ww.w, n, k))
+        torch.cuda.synchronize()
+    be.status_poll()
+    assert not torch.equal(ref[0], ref[1])
+    assert all(torch.equal(y, ref[i % 2]) for i, y in enumerate(ys))
