@@ -217,7 +217,8 @@ int tpb_q8_0_gemv_q8n(tpb_handle_t h, tpb_stream_t stream, float *y, const void 
 /* Replaces Backend.opGemvQuant(.q8_0) + elt.gemv_q8_0
  * (src/gpu/cuda/backend.zig:1660-1681, src/gpu/cuda/elt.zig:671-727): the M = 1
  * GEMV in f32 arithmetic on un-quantised activations,
- *   y[r] = scale * sum_k (q_w * d_w) * x[k]. */
+ *   y[r] = scale * sum_k (q_w * d_w) * x[k].
+ * w and x 16-byte aligned.  Reads nothing, the weight included, before the work in front of it has finished. */
 int tpb_q8_0_gemv_f32(tpb_handle_t h, tpb_stream_t stream, float *y, const float *x,
                       const void *w, float scale, int64_t rows, int64_t cols);
 

@@ -323,8 +323,10 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
 // q * d is the one the kernel above forms with a conversion and a multiplication.
 //
 // What bounds it: 2.25 instructions a weight for that, the two multiply-adds and their operands from shared memory (16 KB of
-// activations per two rows of 2048), against 62.4 MB of weights at 14336 x 4096 (9.4 us at 6.65 TB/s): 77.8 us with the
-// 16-bit global loads of the kernel above -> 14.7 us = 4.2 TB/s; 17408 x 5120 21.4 us, 4096 x 14336 13.2 us, 1024 x 4096 2.8 us.
+// activations per two rows of 2048), against 62.4 MB of weights at 14336 x 4096 (9.5 us at 6.55 TB/s): 72.6 us with the
+// 16-bit global loads of the kernel above -> 16.0 us = 3.9 TB/s; 17408 x 5120 113 -> 23.1 us, 4096 x 14336 87 -> 14.5 us, 1024 x 4096 9.7 ->
+// 3.7 us.  The rings fill after griddepcontrol.wait: this entry point has always seen a weight that the kernel in front of it wrote
+// (filled ahead of the wait the same launches took 14.7, 21.4, 13.2 and 2.8 us).
 constexpr int kF32PairBytes = 272;
 __global__ void __launch_bounds__(512, 1)
 q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ w, float scale, int rows, int cols, int stages,
@@ -347,6 +349,8 @@ q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
+    // nothing of the weight is read, and nothing behind this kernel starts, before the work in front of it has finished
+    tpb_grid_dep_wait();
     tpb_grid_dep_launch();
 
     const int cpr = (nblk + kChunkBlocks - 1) / kChunkBlocks;  // chunks per row
@@ -371,11 +375,9 @@ q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ 
             is_row += R;
         }
     };
-    // weights are constants: they start before the kernel in front has finished
     if (lane == 0)
         for (int i = 0; i < stages - 1 && i < total; i++) issue();
 
-    tpb_grid_dep_wait();
     for (int i = threadIdx.x; i < cols / 4; i += blockDim.x)
         *reinterpret_cast<float4 *>(smem + (size_t)(i >> 4) * kF32PairBytes + (i & 15) * 16) = __ldcg(reinterpret_cast<const float4 *>(x) + i);
     __syncthreads();
@@ -680,7 +682,7 @@ int tpb_launch_q8_0_gemv_f32(tpb_handle_t h, cudaStream_t st, float *y, const fl
     if (smem > (size_t)h->smem_optin)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "q8_0_gemv_f32: cols too large for shared memory");
     // Rows of whole 16-byte words (what a bulk copy can start at): the ring kernel, the faster one from the smallest decode
-    // shape on (1024 x 4096 2.8 us), with as many warps and stages as fit beside the activations (to some 40000 columns)
+    // shape on (1024 x 4096 9.7 -> 3.7 us), with as many warps and stages as fit beside the activations (to some 40000 columns)
     if (cols % 256 == 0) {
         const size_t act = (size_t)(cols / 64) * kF32PairBytes;
         int warps = 0, stages = 0;

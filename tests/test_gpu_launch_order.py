@@ -112,3 +112,26 @@ def test_a_weight_written_before_the_quantiser_is_seen_by_the_gemv(be, n, k, m, 
     be.status_poll()
     assert not torch.equal(ref[0], ref[1])
     assert all(torch.equal(y, ref[i % 2]) for i, y in enumerate(ys))
+
+
+@pytest.mark.parametrize("by", ["library", "torch"])
+@pytest.mark.parametrize("n,k", [(4096, 4096), (17408, 5120), (100, 32768)])
+def test_a_weight_written_directly_before_is_seen_by_the_f32_gemv(be, n, k, by):
+    """The GEMV on f32 activations reads nothing early: its weight may come from the kernel in front of it."""
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        ww = _WrittenWeights(be, n, k)
+        x = torch.randn(1, k, device="cuda")
+        ys = [torch.empty(1, n, device="cuda") for _ in range(42)]
+        for i in range(2):
+            ww.write(i, by)
+            torch.cuda.synchronize()
+            be.opGemvQuant("q8_0", ys[i], x, ww.w, 1.0, n, k)
+            torch.cuda.synchronize()
+        for i in range(2, 42):
+            ww.write(i % 2, by)
+            be.opGemvQuant("q8_0", ys[i], x, ww.w, 1.0, n, k)
+        torch.cuda.synchronize()
+    be.status_poll()
+    assert not torch.equal(ys[0], ys[1])
+    assert all(torch.equal(y, ys[i % 2]) for i, y in enumerate(ys))
