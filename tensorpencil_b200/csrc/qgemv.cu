@@ -282,6 +282,27 @@ q8_1_quantize_kernel(const float *x, float *d, int8_t *qs, int nblk) {
     if (lane == 0) d[blk] = __fdiv_rn(amax, 127.0f);
 }
 
+// One row of the GEMV below by one warp, block b by lane b % 32; ld loads 16 bits of the weight, x(e) is activation e.  Every lane has the sum.
+template <typename Ld, typename X>
+__device__ __forceinline__ float q8_0_row_dot(const uint8_t *wrow, int nblk, int lane, Ld ld, X x) {
+    float acc = 0.0f;
+    for (int b = lane; b < nblk; b += 32) {
+        const unsigned short *blk = reinterpret_cast<const unsigned short *>(wrow + (size_t)b * kBlockBytes);
+        const float dw = __half2float(__ushort_as_half(ld(blk)));
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const unsigned short two = ld(blk + 1 + j);
+            const float q0 = (float)(signed char)(two & 0xff);
+            const float q1 = (float)(signed char)(two >> 8);
+            acc = fmaf(q0 * dw, x(b * 32 + 2 * j), acc);
+            acc = fmaf(q1 * dw, x(b * 32 + 2 * j + 1), acc);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    return acc;
+}
+
 // M = 1 GEMV in f32 arithmetic on un-quantised activations
 // (src/gpu/cuda/elt.zig:671-727): one warp per row, x staged in shared memory.
 __global__ void __launch_bounds__(256)
@@ -295,23 +316,8 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
     for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < rows; row += gridDim.x * wpb) {
-        const uint8_t *wrow = w + (size_t)row * nblk * kBlockBytes;
-        float acc = 0.0f;
-        for (int b = lane; b < nblk; b += 32) {
-            const unsigned short *blk = reinterpret_cast<const unsigned short *>(wrow + (size_t)b * kBlockBytes);
-            const float dw = __half2float(__ushort_as_half(__ldg(blk)));
-            const float *xb = sx + b * 32;
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const unsigned short two = __ldg(blk + 1 + j);
-                const float q0 = (float)(signed char)(two & 0xff);
-                const float q1 = (float)(signed char)(two >> 8);
-                acc = fmaf(q0 * dw, xb[2 * j], acc);
-                acc = fmaf(q1 * dw, xb[2 * j + 1], acc);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        const float acc = q8_0_row_dot(w + (size_t)row * nblk * kBlockBytes, nblk, lane, [](const unsigned short *p) { return __ldg(p); },
+                                       [&](int e) { return sx[e]; });
         if (lane == 0) y[row] = acc * scale;
     }
 }
@@ -320,9 +326,11 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
 // lane takes a block pair of both rows per stage.  f32 activations sit in shared memory, 64 of them every 272 bytes: 16-byte reads
 // at that lane stride fall on distinct banks.  A weight is (32768 + u) * d - 32896 * d in one FMA, u = q + 128 put into
 // the mantissa of 32768 by a byte permute: every step of it is exact (27 bits before, 18 after the FMA's one rounding), so the product
-// q * d is the one the kernel above forms with a conversion and a multiplication.
+// q * d is the one the kernel above forms with a conversion and a multiplication -- but of an infinite d, where it is NaN instead of
+// +-inf.  Rows that come out as NaN are therefore summed again at the end, as the kernel above does it (a branch on
+// infinite scales in the loop cost every row 2-4 %).
 //
-// What bounds it: 2.25 instructions a weight for that, the two multiply-adds and their operands from shared memory (16 KB of
+// What bounds it: 2.25 instructions a weight for that, the two multiply-adds and their operands from shared memory (8 KB of
 // activations per two rows of 2048), against 62.4 MB of weights at 14336 x 4096 (9.5 us at 6.55 TB/s): 72.6 us with the
 // 16-bit global loads of the kernel above -> 16.0 us = 3.9 TB/s; 17408 x 5120 113 -> 23.1 us, 4096 x 14336 87 -> 14.5 us, 1024 x 4096 9.7 ->
 // 3.7 us.  The rings fill after griddepcontrol.wait: this entry point has always seen a weight that the kernel in front of it wrote
@@ -383,6 +391,7 @@ q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ 
     __syncthreads();
 
     f2 acc[R] = {};
+    bool nan = false;
     int st = 0, c = 0, row0 = my_r0;
     uint32_t par = 0;
     for (int i = 0; i < total; i++) {
@@ -448,6 +457,7 @@ q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ 
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
                 if (lane == 0 && row0 + r < my_r1) y[row0 + r] = v * scale;
+                nan |= isnan(v);      // the same in all lanes
                 acc[r] = 0ull;
             }
             c = 0;
@@ -459,6 +469,14 @@ q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ 
             st = 0;
             par ^= 1u;
         }
+    }
+    if (!nan) return;
+    __syncwarp();      // lane 0's results, for all lanes
+    for (int row = my_r0; row < my_r1; row++) {
+        if (!isnan(__ldcg(y + row))) continue;
+        const float v = q8_0_row_dot(w + (size_t)row * row_bytes, nblk, lane, [](const unsigned short *p) { return __ldcg(p); },
+                                     [&](int e) { return *reinterpret_cast<const float *>(smem + (size_t)(e >> 6) * kF32PairBytes + (e & 63) * 4); });
+        if (lane == 0) y[row] = v * scale;
     }
 }
 

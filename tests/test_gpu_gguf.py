@@ -201,3 +201,26 @@ def test_gguf_gemv_large_weights_give_the_same_bits_on_every_kernel(be, fmt, n, 
     for kern in ("mma", "warp"):
         monkeypatch.setenv("TPB_GEMVK_KERNEL", kern)
         assert np.array_equal(auto, run(be, fmt, w, n, k, x)), kern
+
+
+@pytest.mark.parametrize("k", [96, 256, 4096])
+def test_q8_0_gemv_f32_with_infinite_block_scales(be, k):
+    """q * d with an infinite d is +-inf, or NaN where q is 0, on every kernel behind the entry point: a row is then +-inf, or NaN where
+    infinities of both signs or such a NaN meet.  The other rows of a row pair keep their finite results."""
+    n = 9
+    w = synth.gguf_weights("q8_0", n, k, seed=k).reshape(n, k // 32, 34).copy()
+    x = np.random.default_rng(k).uniform(0.5, 1.5, k).astype(np.float32)
+    inf = {1: (0, 0x7c00, 5), 2: (k // 32 - 1, 0xfc00, 5), 4: (k // 64, 0x7c00, 0), 7: (0, 0x7c00, None), 8: (k // 32 - 1, 0xfc00, -3)}
+    for r, (b, d, q) in inf.items():                     # row -> block, its f16 scale, its quants (None: as they are, of both signs)
+        w[r, b, :2] = np.frombuffer(np.uint16(d).tobytes(), np.uint8)
+        if q is not None:
+            w[r, b, 2:] = np.int8(q).view(np.uint8)
+    w = w.reshape(n, -1)
+    y = torch.empty(n, dtype=torch.float32, device="cuda")
+    be.opGemvQuant("q8_0", y, torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), 1.0, n, k)
+    be.status_poll()
+    got = y.cpu().numpy()
+    assert got[1] == np.inf and got[2] == -np.inf and np.isnan(got[4]) and np.isnan(got[7]) and got[8] == np.inf
+    rest = [r for r in range(n) if r not in inf]
+    wf = np.stack([oracle.q8_0_dequant_row(w[r], k) for r in rest]).astype(np.float64)
+    assert np.allclose(got[rest], wf @ x.astype(np.float64), rtol=0, atol=1e-5 * float((np.abs(wf) @ x).max()))
