@@ -332,8 +332,8 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
 //
 // What bounds it: 2.25 instructions a weight for that, the two multiply-adds and their operands from shared memory (8 KB of
 // activations per two rows of 2048), against 62.4 MB of weights at 14336 x 4096 (9.5 us at 6.55 TB/s): 72.6 us with the
-// 16-bit global loads of the kernel above -> 16.0 us = 3.9 TB/s; 17408 x 5120 113 -> 23.1 us, 4096 x 14336 87 -> 14.5 us, 1024 x 4096 9.7 ->
-// 3.7 us.  The rings fill after griddepcontrol.wait: this entry point has always seen a weight that the kernel in front of it wrote
+// 16-bit global loads of the kernel above -> 16.2 us = 3.9 TB/s; 17408 x 5120 113 -> 23.5 us, 4096 x 14336 87 -> 14.6 us, 1024 x 4096 9.7 ->
+// 3.6 us.  The rings fill after griddepcontrol.wait: this entry point has always seen a weight that the kernel in front of it wrote
 // (filled ahead of the wait the same launches took 14.7, 21.4, 13.2 and 2.8 us).
 constexpr int kF32PairBytes = 272;
 __global__ void __launch_bounds__(512, 1)
@@ -699,15 +699,16 @@ int tpb_launch_q8_0_gemv_f32(tpb_handle_t h, cudaStream_t st, float *y, const fl
     const size_t smem = (size_t)cols * 4;
     if (smem > (size_t)h->smem_optin)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "q8_0_gemv_f32: cols too large for shared memory");
-    // Rows of whole 16-byte words (what a bulk copy can start at): the ring kernel, the faster one from the smallest decode
-    // shape on (1024 x 4096 9.7 -> 3.7 us), with as many warps and stages as fit beside the activations (to some 40000 columns)
-    if (cols % 256 == 0) {
+    // Rows of whole 16-byte words (what a bulk copy can start at) from 1024 columns on: the ring kernel, with as many warps as fit beside
+    // the activations (to some 40000 columns).  Shorter rows leave most lanes of its warps without a block, a few rows one or two CTAs, and
+    // the plain kernel starts faster: us, plain / ring: 64 x 256 1.9 / 2.6, 16 x 512 2.4 / 3.0, 2048 x 512 3.15 / 3.12; 16 x 1024 3.3 / 3.5,
+    // 64 x 1024 3.25 / 3.05, 16 x 2048 5.3 / 3.5, 1024 x 1024 3.4 / 2.4.
+    // Two stages at every size: 4096 x 4096 7.1 us with four, 6.3 with two, 14336 x 4096 16.8 / 16.0, 1024 x 4096 3.7 / 3.6, the other
+    // shapes within 1 %.
+    if (cols % 256 == 0 && cols >= (rows < 64 ? 2048 : 1024)) {
         const size_t act = (size_t)(cols / 64) * kF32PairBytes;
         int warps = 0, stages = 0;
-        // two stages from 16 MB on: 4096 x 4096 6.2 -> 5.5 us, 5120 x 5120 10.7 -> 9.9, 14336 x 4096 15.4 -> 14.7, 32000 x 4096
-        // 25.3 -> 24.2; below, deeper rings bring most of the weight in at once: 1024 x 4096 2.8 us against 3.6, 3072 x 3072 4.7 / 5.8
-        const int max_stages = (double)rows * (double)(cols / 32) * kBlockBytes >= 16e6 ? 2 : 4;
-        dp4a_plan(h, act, rows, stage_bytes(2), 16, max_stages, &warps, &stages);
+        dp4a_plan(h, act, rows, stage_bytes(2), 16, 2, &warps, &stages);
         if (warps != 0) {
             int rgrid = (int)((rows + 2 * warps - 1) / (2 * warps));
             if (rgrid > h->sm_count) rgrid = h->sm_count;

@@ -158,7 +158,7 @@ def test_q6k_weight_at_the_very_end_of_its_allocation(be):
     assert np.array_equal(y.cpu().numpy(), want)
 
 
-@pytest.mark.parametrize("n,k", [(1, 256), (7, 768), (33, 2304), (300, 4096), (2500, 1024), (149, 17408), (20, 32768), (9, 96)])
+@pytest.mark.parametrize("n,k", [(1, 256), (7, 768), (33, 2304), (63, 1024), (64, 1024), (300, 4096), (2500, 1024), (149, 17408), (20, 32768), (9, 96)])
 def test_q8_0_gemv_f32_at_the_edges_of_its_rings(be, n, k):
     """The single-row GEMV on f32 activations: one row, odd rows per warp, rows of less than a chunk, a chunk and a bit, many chunks,
     the activations that leave the fewest rings, and a row length that bulk copies cannot take (the plain kernel)."""
