@@ -528,14 +528,17 @@ static void dp4a_plan(tpb_handle_t h, size_t act, int64_t rows, int stage, int m
     }
 }
 
-// Ring depth of the dp4a kernel.  A warp's copies are issued by its first lane between two steps of arithmetic, and where a warp has few
-// steps the copies of a third and fourth stage delay them more than they save: us at M = 1, 2, 4 with up to four stages / with two:
-// 4096 x 4096 5.3 5.7 7.0 / 4.7 5.2 6.3, 5120 x 5120 8.5 9.5 11.3 / 8.1 8.8 10.9, 11008 x 4096 9.8 10.5 13.3 / 9.6 10.0 12.6, 4096 x 11008
-// 10.1 11.1 13.0 / 9.8 10.6 13.0.  Not for short rows (9216 x 2304 7.3 / 7.5), small weights (1024 x 5120 3.6 / 4.4) or many
-// steps (14336 x 4096 11.7 / 12.2, 8192 x 8192 12.2 / 12.6).
-static int q8n_stages(int64_t rows, int64_t cols) {
+// Ring depth of the dp4a kernel: two stages where the one that is on its way while a warp works on the other covers the memory's latency,
+// four where it does not.  Sixteen warps with a stage of two whole chunks (4.3 KB) on its way are 70 KB per SM, 10 MB in all, and HBM
+// needs some 6.5 MB (1 us at 6.55 TB/s); what a deeper ring adds is copies that a warp's first lane issues between two steps of
+// arithmetic.  us at M = 1, 2, 4 with up to four stages / with two: 4096 x 4096 5.3 5.7 7.1 / 4.6 5.2 6.5, 5120 x 5120 8.5 9.4 11.2 / 7.9
+// 8.7 10.8, 11008 x 4096 10.1 11.0 13.5 / 9.7 10.4 13.0, 4096 x 11008 10.4 11.4 13.2 / 10.2 10.8 13.1.  With fewer than one and a half rows a
+// warp the stages hold one row, and with short rows their last chunk, too little: 1024 x 4096 2.7 3.2 3.9 / 3.2 3.6 4.5, 1500 x 14336 8.8 9.8
+// 12.7 / 10.5 10.0 12.7, 3000 x 11264 9.3 9.8 11.8 / 10.5 9.0 11.3, 9216 x 2304 7.3 8.0 9.6 / 7.4 8.1 9.8.  From 56 MB on the two differ by
+// 1 % either way at M = 1 (14336 x 4096 12.3 / 12.4, 8192 x 8192 13.0 / 13.1).
+static int q8n_stages(tpb_handle_t h, int64_t rows, int64_t cols) {
     const double bytes = (double)rows * (double)(cols / 32) * kBlockBytes;
-    return cols >= 4096 && bytes >= 16e6 && bytes < 56e6 ? 2 : 4;
+    return cols >= 4096 && rows >= 24 * h->sm_count && bytes < 56e6 ? 2 : 4;
 }
 
 template <int M, int R>
@@ -557,7 +560,7 @@ int launch_q8n_cfg(tpb_handle_t h, cudaStream_t st, const GemvParams &p, int max
         TPB_CUDA(h, launch_pdl(kern, grid, ov.warps * 32, need, st, p, ov.stages));
         return TPB_OK;
     }
-    dp4a_plan(h, act, p.rows, kStage, max_warps, q8n_stages(p.rows, p.cols), &warps, &stages);
+    dp4a_plan(h, act, p.rows, kStage, max_warps, q8n_stages(h, p.rows, p.cols), &warps, &stages);
     if (stages == 0) {
         if (R == 2) return TPB_ERR_STATE;
         act_smem = false;
@@ -646,7 +649,7 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
             // the dp4a kernel at its best: fourteen warps with two two-row stages each fit beside the activations
             // (with fewer its time jumps: K = 14336 from the sixth activation row on, K = 28672 from the third)
             int warps = 0, stages = 0;
-            dp4a_plan(h, act_bytes, rows, stage_bytes(2), 16, q8n_stages(rows, cols), &warps, &stages);
+            dp4a_plan(h, act_bytes, rows, stage_bytes(2), 16, q8n_stages(h, rows, cols), &warps, &stages);
             const bool roomy = warps != 0 && act_bytes + 14 * 2 * (size_t)stage_bytes(2) + 14 * 2 * 8 + 64 <=
                                                  (size_t)h->smem_optin - 1024;
             // share of its row slots that hold a row: rows come to a warp two at a time

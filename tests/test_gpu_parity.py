@@ -353,6 +353,21 @@ def test_q8_0_gemv_long_rows(be, monkeypatch, m, n, k, route):
     assert np.max(np.abs(y - want)) <= tol, (np.max(np.abs(y - want)), tol)
 
 
+@pytest.mark.parametrize("m", [1, 2, 4])
+@pytest.mark.parametrize("n,k", [(3551, 4096), (3552, 4096), (3552, 4064), (3600, 13824), (13160, 4096), (1024, 5120)])
+def test_q8_0_gemv_ring_depth_does_not_change_a_bit(be, monkeypatch, m, n, k):
+    """Both sides of each line of the ring depth's rule (rows per warp, columns, bytes) against eight warps with three stages."""
+    g = synth.q8_0_gemv(m, n, k, seed=n + m)
+    x = dev(g["x"])
+    monkeypatch.setenv("TPB_GEMV_KERNEL", "dp4a")
+    y = be.q8_0_linear(x, g["w"], n, k)
+    monkeypatch.setenv("TPB_GEMV_CFG", "2,8,3")
+    want = be.q8_0_linear(x, g["w"], n, k)
+    be.status_poll()
+    be.dropWeights()
+    assert torch.equal(y, want)
+
+
 def test_q8_0_gemv_more_than_8_rows_groups(be):
     g = synth.q8_0_gemv(19, 32, 1024, seed=5)
     y = be.q8_0_linear(dev(g["x"]), g["w"], 32, 1024).cpu().numpy()
