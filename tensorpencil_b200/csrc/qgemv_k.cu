@@ -847,21 +847,85 @@ static int k_kernel_override() {
     return e[0] == 'r' ? 1 : e[0] == 'w' ? 2 : e[0] == 'm' ? 3 : 0;
 }
 
+// Shared memory of the dp4a kernels: the activations of ng rows, and one stage of a warp's ring (two weight rows).
+static size_t kq_act_bytes(int fmt, int ng, int64_t cols) {
+    return (size_t)ng * (size_t)(cols / 64) * kActPairBytes + (size_t)ng * (size_t)(cols / 32) * (fmt == TPB_GGUF_Q6_K ? 12 : 8);
+}
+// Three 64-element units per lane and chunk where that takes fewer chunks per row than two (launch_fmt_m).
+static bool kq_three_units(int ng, int64_t cols) {
+    const int64_t n_units = cols / 64;
+    return ng <= 4 && (n_units + 95) / 96 < (n_units + 63) / 64;
+}
+static size_t kq_stage_bytes(int fmt, int ng, int64_t cols) {
+    if (fmt == TPB_GGUF_Q6_K) return 2 * (size_t)kQ6RowStage;
+    return 2 * (size_t)32 * (kq_three_units(ng, cols) ? 3 : 2) * (fmt == TPB_GGUF_Q5_K ? 44 : 36);
+}
+// Warps per CTA: every warp owns a contiguous range of whole rows; among the counts that fit with >= 2 stages take the one whose
+// ranges divide most evenly (ties: more warps).
+static void kq_plan(tpb_handle_t h, size_t act, size_t stage, int64_t rows, int max_stages, int *warps, int *stages) {
+    const size_t limit = (size_t)h->smem_optin - 1024;
+    *warps = *stages = 0;
+    double best_eff = -1.0;
+    for (int w = 16; w >= 4; w--) {
+        int s_fit = 0;
+        for (int s = max_stages; s >= 2; s--)
+            if (act + (size_t)w * s * stage + (size_t)w * s * 8 + 64 <= limit) {
+                s_fit = s;
+                break;
+            }
+        if (s_fit == 0) continue;
+        const double per_warp = (double)rows / ((double)h->sm_count * w);
+        const double eff = per_warp >= 1.0 ? per_warp / (double)(long long)(per_warp + 0.999999) : per_warp;
+        if (eff > best_eff + 0.02) {
+            best_eff = eff;
+            *warps = w;
+            *stages = s_fit;
+        }
+    }
+}
+
+// Ring depth of the dp4a kernel of q4_0, iq4_nl, q4_k and q5_k: two stages from 14 MB on.  A warp's copies are issued by its first lane
+// between two steps of arithmetic, and once a stage of two rows per warp covers the memory's latency those of a third and fourth only
+// delay the steps.  us at M = 1, 2, 4, up to four stages / two: 14336 x 4096 q4_0 10.0 11.3 15.0 / 9.3 10.6 14.5, iq4_nl 17.1 18.2 21.9 / 16.5 17.6
+// 21.4, q4_k 10.4 11.9 15.1 / 9.7 11.3 14.7; 5120 x 5120 q4_k 7.8 8.5 10.6 / 7.2 8.0 10.3, q5_k 8.7 9.6 12.2 / 8.2 9.2 11.7.  Below, the two are within
+// 2 % but for 2048 x 8192 (q4_k 5.5 / 5.6 at M = 1).  The q6_k kernel keeps up to four.
+static int kq_max_stages(int64_t rows, size_t row_bytes) { return (double)rows * (double)row_bytes >= 14e6 ? 2 : 4; }
+
 // Whether the mma.sync kernel (qgemv_kmma.cu: the same bits, nearly the same time for any number of activation rows) beats the
-// dp4a kernels, whose time grows by 10-20 % with every row and, on long rows, jumps where the activations crowd the rings out or
-// the group has to be split.  Measured on ten shapes and five formats; us, dp4a / mma, q4_k unless said:
-//   M = 8   1024 x 4096 6.1 / 6.5 (q4_0)   1024 x 5120 8.2 / 7.2   4096 x 4096 8.5 / 8.0   14336 x 4096 22.2 / 15.0
-//   M = 5   4096 x 4096 6.8 / 7.7   9216 x 2304 9.6 / 9.3   2048 x 8192 9.6 / 8.0   5120 x 5120 13.5 / 10.1   17408 x 5120 24.0 / 17.6
-//   M = 4   4096 x 4096 6.2 / 7.6   9216 x 2304 8.6 / 9.2   2048 x 8192 8.4 / 7.7   5120 x 5120 10.6 / 9.9   14336 x 4096 15.2 / 14.5
-//           17408 x 5120 19.1 / 17.5 (q6_k 31.3 / 28.5)   5120 x 17408 26.4 / 26.0 (q5_k 30.4 / 28.2, q6_k 41.4 / 40.4)
-//   M = 3   17408 x 5120 16.9 / 17.7   32000 x 4096 30.0 / 22.8 (q6_k 34.4 / 33.9)
-static bool mma_wins(int64_t rows, int64_t cols, int m) {
+// dp4a kernels, whose time grows by 10-20 % with every row.  The line between them follows a measurement of five formats over 28 row
+// counts from 1000 to 32000 and nine column counts from 2048 to 17408 (us, dp4a / mma):
+//   few    the dp4a kernel's plan comes down to five warps or fewer (rows that divide badly, or activations that crowd the rings out), too
+//          few to keep an SM busy: M = 4 13500 x 8192 q4_k 36.7 / 24.4, 10000 x 5120 q6_k 33.2 / 20.5; M = 3 32000 x 4096 q4_k 30.0 / 23.4
+//   fill   the share of the mma kernel's 16-row groups that holds a row: 2500 rows are 17 per SM, two groups.  M = 5 2500 x 14336 q4_k 14.1 / 16.6
+//   best   the dp4a kernel's best: fourteen warps or more whose two-row stages are all full.  M = 5 12288 x 8192 q4_k 22.8 / 24.3, 9216 x 4096
+//          10.5 / 10.9
+//   M = 4  even but for rows that leave the dp4a kernel's last chunk part empty: 17408 x 5120 q4_k 19.6 / 17.9, q5_k 25.3 / 22.1, 5120 x 17408 q4_k
+//          26.9 / 25.5, but 3072 x 17408 q5_k 21.6 / 22.4; whole chunks 8192 x 8192 q4_k 14.7 / 16.3, 4096 x 6144 q4_k 7.8 / 9.6; q6_k 12288 x 8192 30.9 / 40.4, 5120 x 17408 41.8 / 41.1
+//   M = 5  17408 x 5120 q4_k 24.3 / 18.4, 2000 x 8192 9.6 / 8.3; M = 6 7000 x 4096 11.0 / 11.4; q6_k at K = 8192 (two passes) 12288 rows 35.4 / 40.8, 17408 44.5 / 51.0
+//   K < 4096  two or three units per warp and row group: 12288 x 2048 q4_k M = 5 9.2 / 10.4, M = 6 10.1 / 10.5, 4096 x 2048 M = 8 6.0 / 6.6
+//   M = 8  1000 x 5120 q4_k 8.2 / 7.2, 4096 x 4096 8.5 / 8.1, 14336 x 4096 22.1 / 14.9
+static bool mma_wins(tpb_handle_t h, int fmt, int64_t rows, int64_t cols, int m) {
     const int64_t weights = rows * cols;
-    if (m >= 4 && cols >= 8192) return weights >= 16000000;
-    if (m == 8) return weights >= (cols >= 5120 ? 5000000 : 8000000);
-    if (m >= 5) return weights >= 20000000;
-    if (m == 4) return cols >= 4096 && weights >= 25000000;
-    return m == 3 && cols >= 4096 && weights >= 120000000;
+    if (m < 3 || weights < 5000000) return false;
+    int warps = 0, stages = 0;
+    const int max_stages = fmt == TPB_GGUF_Q6_K ? 4 : kq_max_stages(rows, tpb_gguf_row_bytes(fmt, cols));
+    kq_plan(h, kq_act_bytes(fmt, m, cols), kq_stage_bytes(fmt, m, cols), rows, max_stages, &warps, &stages);
+    if (warps <= 5 && weights >= 20000000) return true;
+    const double per_cta = (double)rows / h->sm_count > 4.0 ? (double)rows / h->sm_count : 4.0;
+    const double fill = per_cta / (16.0 * (double)((long long)(per_cta / 16.0 + 0.999999)));
+    if (m == 3 || fill < 0.6) return false;
+    if (m == 4) {
+        const int64_t chunk = kq_three_units(m, cols) ? 96 * 64 : 64 * 64;
+        return fmt != TPB_GGUF_Q6_K && cols >= 5120 && cols % chunk != 0 && rows >= 5000 && weights >= 44000000 && (fill >= 0.88 || warps <= 7);
+    }
+    if (m == 8) return weights >= (cols >= 5120 ? 5000000 : cols >= 4096 ? 8000000 : 16000000);
+    if (m == 5) {
+        const double pairs = warps ? (double)rows / ((double)h->sm_count * warps * 2) : 0.0;
+        const bool best = warps >= 14 && pairs >= 0.95 * (double)((long long)(pairs + 0.999999));
+        if (best || (fmt == TPB_GGUF_Q6_K && cols >= 8192 && cols % 4096 == 0)) return false;
+    }
+    if (cols < 4096) return weights >= (m == 5 ? 60000000 : m == 6 ? 40000000 : 20000000);
+    return weights >= (cols >= 8192 ? 16000000 : m == 6 ? 30000000 : 20000000);
 }
 
 template <int M>
@@ -892,26 +956,9 @@ int launch_q6k_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
         if (s_r >= 3 && (force == 1 || (force == 0 && pick))) return launch_q6k_ring<M>(h, st, p, s_r > 12 ? 12 : s_r, act_r);
     }
     constexpr int kStage = R * kQ6RowStage;
-    const size_t limit = (size_t)h->smem_optin - 1024;
-    const size_t act = (size_t)M * (p.cols / 64) * kActPairBytes + (size_t)M * p.nblk * 4 + (size_t)M * (p.cols / 16) * 4;
+    const size_t act = kq_act_bytes(TPB_GGUF_Q6_K, M, p.cols);
     int warps = 0, stages = 0;
-    double best_eff = -1.0;
-    for (int w = 16; w >= 4; w--) {
-        int s_fit = 0;
-        for (int s = 4; s >= 2; s--)
-            if (act + (size_t)w * s * kStage + (size_t)w * s * 8 + 64 <= limit) {
-                s_fit = s;
-                break;
-            }
-        if (s_fit == 0) continue;
-        const double per_warp = (double)p.rows / ((double)h->sm_count * w);
-        const double eff = per_warp >= 1.0 ? per_warp / (double)(long long)(per_warp + 0.999999) : per_warp;
-        if (eff > best_eff + 0.02) {
-            best_eff = eff;
-            warps = w;
-            stages = s_fit;
-        }
-    }
+    kq_plan(h, act, kStage, p.rows, 4, &warps, &stages);
     if (stages == 0)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "gguf_gemv: %d activation rows of %d columns do not fit shared memory",
                         M, p.cols);
@@ -944,33 +991,9 @@ template <int FMT, int M, int U>
 int launch_fmt_mu(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     constexpr int R = 2;
     constexpr int kStage = R * 32 * U * Fmt<FMT>::kUnitBytes;
-    const size_t limit = (size_t)h->smem_optin - 1024;
     const size_t act = (size_t)M * (p.cols / 64) * kActPairBytes + (size_t)M * p.nblk * 8;
-    // Warps per CTA: every warp owns a contiguous range of whole rows; among the counts that
-    // fit with >= 2 stages take the one whose ranges divide most evenly (ties: more warps).
-    // Two stages per ring from 14 MB on: a warp's copies are issued by its first lane between two steps of arithmetic, and those of a
-    // third and fourth stage delay the few steps there are.  us at M = 1, 2, 4, up to four stages / two: q4_k 14336 x 4096 10.6 12.0
-    // 15.2 / 9.8 11.3 14.7, 5120 x 5120 7.8 8.6 10.6 / 7.3 8.2 10.3; q5_k 5120 x 5120 8.6 9.8 12.2 / 8.2 9.2 11.7.  Below, deeper rings bring more
-    // of a small weight in at once (q4_k 2048 x 8192 5.5 / 5.7 at M = 1).
-    const int max_stages = (double)p.rows * (double)p.row_bytes >= 14e6 ? 2 : 4;
     int warps = 0, stages = 0;
-    double best_eff = -1.0;
-    for (int w = 16; w >= 4; w--) {
-        int s_fit = 0;
-        for (int s = max_stages; s >= 2; s--)
-            if (act + (size_t)w * s * kStage + (size_t)w * s * 8 + 64 <= limit) {
-                s_fit = s;
-                break;
-            }
-        if (s_fit == 0) continue;
-        const double per_warp = (double)p.rows / ((double)h->sm_count * w);
-        const double eff = per_warp >= 1.0 ? per_warp / (double)(long long)(per_warp + 0.999999) : per_warp;
-        if (eff > best_eff + 0.02) {
-            best_eff = eff;
-            warps = w;
-            stages = s_fit;
-        }
-    }
+    kq_plan(h, act, kStage, p.rows, kq_max_stages(p.rows, p.row_bytes), &warps, &stages);
     if (stages == 0)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "gguf_gemv: %d activation rows of %d columns do not fit shared memory",
                         M, p.cols);
@@ -1023,7 +1046,7 @@ int launch_fmt_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     // (q5_k, M = 8: 38 -> 45 us), so only up to four
     const int n_units = p.cols / 64;
     bool u3 = false;
-    if constexpr (M <= 4) u3 = (n_units + 95) / 96 < (n_units + 63) / 64;
+    if constexpr (M <= 4) u3 = kq_three_units(M, p.cols);
     // The ring kernel for one or two activation rows where the per-warp rings serialise: rows of several chunks
     // (K = 17408, M = 1: q4_k 21.5 -> 14.4 us, q4_0 18.2 -> 12.7, q5_k 25.1 -> 18.2) and many rows per warp
     // (32000 x 4096: q4_k 28.9 -> 19.2 us).  With short rows and few of them per warp the two are within 5 %
@@ -1067,15 +1090,7 @@ int launch_fmt(tpb_handle_t h, cudaStream_t st, const KGemvParams &p, int ng) {
 // stages each) of the format's kernel.
 bool kq_group_fits(tpb_handle_t h, int fmt, int ng, int64_t cols) {
     const size_t limit = (size_t)h->smem_optin - 1024;
-    const size_t n_units = (size_t)(cols / 64), nblk = (size_t)(cols / 32);
-    const size_t act = (size_t)ng * n_units * kActPairBytes + (size_t)ng * nblk * (fmt == TPB_GGUF_Q6_K ? 12 : 8);
-    size_t stage;
-    if (fmt == TPB_GGUF_Q6_K) {
-        stage = 2 * (size_t)kQ6RowStage;
-    } else {
-        const bool u3 = ng <= 4 && (n_units + 95) / 96 < (n_units + 63) / 64;
-        stage = 2 * (size_t)32 * (u3 ? 3 : 2) * (fmt == TPB_GGUF_Q5_K ? 44 : 36);
-    }
+    const size_t act = kq_act_bytes(fmt, ng, cols), stage = kq_stage_bytes(fmt, ng, cols);
     return act + 4 * 2 * stage + 4 * 2 * 8 + 64 <= limit;
 }
 
@@ -1112,7 +1127,7 @@ int tpb_gguf_gemv_q8n(tpb_handle_t h, tpb_stream_t stream, int fmt, float *y, co
     if (rows == 0) return TPB_OK;
     const int nblk = (int)(cols / 32);
     const int force = k_kernel_override();
-    if ((force == 3 || (force == 0 && mma_wins(rows, cols, ng))) && tpb_kquant_mma_fits(h, fmt, rows, cols))
+    if ((force == 3 || (force == 0 && mma_wins(h, fmt, rows, cols, ng))) && tpb_kquant_mma_fits(h, fmt, rows, cols))
         return tpb_launch_kquant_mma(h, (cudaStream_t)stream, fmt, y, reinterpret_cast<const uint8_t *>(w), scale, rows, cols,
                                      reinterpret_cast<const float *>(xq) + (size_t)row_off * nblk,
                                      reinterpret_cast<const int8_t *>(xq) + (size_t)n_total * nblk * 4 + (size_t)row_off * cols, ng);

@@ -192,7 +192,8 @@ def test_gguf_gemv_mma_kernel_gives_the_dp4a_kernels_bits(be, fmt, m, n, k, monk
 
 
 @pytest.mark.parametrize("m", [3, 4, 5, 8])
-@pytest.mark.parametrize("fmt,n,k", [("q4_k", 5100, 5120), ("q5_k", 2050, 8192), ("q6_k", 1030, 17408), ("iq4_nl", 9001, 2304)])
+@pytest.mark.parametrize("fmt,n,k", [("q4_k", 5100, 5120), ("q5_k", 2050, 8192), ("q6_k", 1030, 17408), ("iq4_nl", 9001, 2304),
+                                     ("q4_k", 3600, 5632), ("q4_0", 2500, 8192), ("q6_k", 4096, 8192)])
 def test_gguf_gemv_large_weights_give_the_same_bits_on_every_kernel(be, fmt, n, k, m, monkeypatch):
     """Shapes on both sides of the dispatch rule; many row groups per CTA."""
     w = synth.gguf_weights(fmt, n, k, seed=n)
