@@ -1127,7 +1127,10 @@ int tpb_gguf_gemv_q8n(tpb_handle_t h, tpb_stream_t stream, int fmt, float *y, co
     if (rows == 0) return TPB_OK;
     const int nblk = (int)(cols / 32);
     const int force = k_kernel_override();
-    if ((force == 3 || (force == 0 && mma_wins(h, fmt, rows, cols, ng))) && tpb_kquant_mma_fits(h, fmt, rows, cols))
+    // rows too long for a single activation row of the dp4a kernel are refused whatever the group (below), also where the mma kernel could
+    // take them
+    if ((force == 3 || (force == 0 && mma_wins(h, fmt, rows, cols, ng))) && kq_group_fits(h, fmt, 1, cols) &&
+        tpb_kquant_mma_fits(h, fmt, rows, cols))
         return tpb_launch_kquant_mma(h, (cudaStream_t)stream, fmt, y, reinterpret_cast<const uint8_t *>(w), scale, rows, cols,
                                      reinterpret_cast<const float *>(xq) + (size_t)row_off * nblk,
                                      reinterpret_cast<const int8_t *>(xq) + (size_t)n_total * nblk * 4 + (size_t)row_off * cols, ng);

@@ -15,6 +15,7 @@ torch = pytest.importorskip("torch")
 
 from oracle import oracle  # noqa: E402
 from tensorpencil_b200 import synth  # noqa: E402
+from tensorpencil_b200._lib import TpbError  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -225,3 +226,14 @@ def test_q8_0_gemv_f32_with_infinite_block_scales(be, k):
     rest = [r for r in range(n) if r not in inf]
     wf = np.stack([oracle.q8_0_dequant_row(w[r], k) for r in rest]).astype(np.float64)
     assert np.allclose(got[rest], wf @ x.astype(np.float64), rtol=0, atol=1e-5 * float((np.abs(wf) @ x).max()))
+
+
+@pytest.mark.parametrize("fmt", ["q4_k", "q6_k"])
+def test_rows_too_long_for_one_activation_row_are_refused_for_every_group(be, fmt):
+    n, k = 80, 1 << 18
+    w = torch.zeros(n * synth.gguf_weights(fmt, 1, k, seed=1).size, dtype=torch.uint8, device="cuda")
+    y = torch.zeros((8, n), dtype=torch.float32, device="cuda")
+    be.opGemvQuantizeX(torch.zeros((8, k), device="cuda"), 8 * k)
+    for m in (1, 3, 4, 5, 8):
+        with pytest.raises(TpbError):
+            be.opGemvQuantQ8N(fmt, y, w, 1.0, n, k, m, 0, 8)
