@@ -83,11 +83,7 @@ __device__ __forceinline__ void w4_expand_chunk(const uint4 *__restrict__ w4, ui
 
 
 constexpr int kMaxWarps = 8;
-constexpr int kMaxWarpsWide = 16;
-#ifndef TPB_F32_LOAD_FIRST
-#define TPB_F32_LOAD_FIRST 1
-#endif
-constexpr bool kF32LoadFirst = TPB_F32_LOAD_FIRST != 0;   // rows of the gated preps: one unit per half-warp, more warps per row
+constexpr int kMaxWarpsWide = 16;   // of a row with one unit per half-warp
 constexpr int kTilePairs = 16 * 18;  // 64-bit slots of one half-warp's tile (2304 bytes)
 constexpr size_t kMaxPrepSmem = (size_t)kMaxWarpsWide * 2 * kTilePairs * 8;   // of the widest row's CTA
 
@@ -500,7 +496,7 @@ convrot_prep_kernel(const PrepParams P) {
 }
 
 // Narrow rows (k <= 1024: one warp's worth) run four rows per CTA, one warp each.  Wider
-// rows take one CTA per row with as many warps as possible (up to 8) and 1..4 group pairs
+// rows take one CTA per row with as many warps as possible (up to 8, or 16: see below) and 1..4 group pairs
 // per half-warp: many warps with few pairs each beat few warps with many (measured at
 // k = 3072 and 12288, also against a persistent grid that prefetches the next row into
 // registers) -- occupancy hides more latency than the per-thread bookkeeping costs.
@@ -521,11 +517,12 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
         const size_t smem = ACT_ONLY ? 0 : (size_t)kRowsPerCta * 2 * kTilePairs * sizeof(f2);
         err = tpb_launch_pdl(convrot_prep_kernel<T, 1, OP, ACT_ONLY, true>, grid, block, smem, st, P);
     } else {
-        // One unit per half-warp, up to 16 warps a row, while the row fits that way (k <= 16384): the warps a row has in flight
-        // hide its latencies, and with two units each they were half as many.  Against 8 warps of two units (us, bf16): SiLU gate
-        // 4608 x 12288 152 -> 82, RMS norm 104 -> 98, 1111 x 9216 21.6 -> 19.5, plain 1111 x 9216 14.1 -> 13.2, 512 x 12288 11.3 -> 10.1,
-        // 4608 x 12288 58.1 -> 57.9.
-        const bool wide = n_units <= 2 * kMaxWarpsWide;
+        // One unit per half-warp, up to 16 warps a row, where the row fits that way (k <= 16384): the warps a row has in flight
+        // hide its latencies, and with two units each they are half as many.  us, 8 warps of two units / one unit each: SiLU gate 4608 x 12288 bf16
+        // 152 / 82, plain f32 1111 x 8448 13.4 / 12.9, 4608 x 13312 78.9 / 74.0, bf16 512 x 12288 11.3 / 10.1, 4608 x 12288 58.1 / 57.9.
+        // RMS norm keeps two units: its sum of squares has always been taken in that order.
+        constexpr bool kGated = OP == OP_SILU_MUL || OP == OP_SIGMOID_MUL;
+        const bool wide = n_units <= 2 * kMaxWarpsWide && (kGated || OP == OP_PLAIN);
         const int max_warps = wide ? kMaxWarpsWide : kMaxWarps;
         const int upw = (n_units + 2 * max_warps - 1) / (2 * max_warps);  // 1..4 for k <= 32768
         const int warps = (n_units + 2 * upw - 1) / (2 * upw);
@@ -539,9 +536,12 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
         if (err == cudaSuccess) err = tpb_launch_pdl(kern, grid, block, smem, st, P);                   \
         break;                                                                                          \
     }
+        if constexpr (!kGated) {      // the gated rows of 17 .. 32 units are wide
+            switch (upw) { TPB_PREP_CASE(2) }
+        }
         switch (upw) {
             TPB_PREP_CASE(1)
-            TPB_PREP_CASE(2)
+            case 2: break;
             TPB_PREP_CASE(3)
             TPB_PREP_CASE(4)
             default: return tpb_fail(h, TPB_ERR_INVALID_ARG, "prep: k = %lld is too wide", (long long)k);

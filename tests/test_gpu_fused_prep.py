@@ -249,6 +249,53 @@ def test_gemm_with_silu_pair_into_a_wider_buffer_and_bad_arguments(be):
     assert L.tpb_convrot_gemm_silu_pair(*args(_lib.TPB_F32, None)) == _lib.TPB_ERR_INVALID_ARG            # second weight missing
 
 
+def _rms_sum_of_squares(row):
+    """The f32 sum of squares of a row in the kernel's order: a half-warp takes pairs of 256-element groups, a lane elements
+    4 (l + 16 i) + j of both; one FMA chain per lane over its units, a butterfly over the warp, the warps in order."""
+    k = row.size
+    n_groups, n_units = k // 256, (k // 256 + 1) // 2
+    if n_units <= 2:
+        warps, upw = 1, 1
+    else:
+        upw = -(-n_units // 16)
+        warps = -(-n_units // (2 * upw))
+    lanes = np.zeros((warps, 2, 16), np.float32)
+    for p in range(upw):
+        for w in range(warps):
+            for hw in range(2):
+                g0 = 2 * ((2 * w + hw) + p * 2 * warps)
+                for i in range(4):
+                    for h in range(2):
+                        if g0 + h < n_groups:
+                            x = row[(g0 + h) * 256 + 64 * i:(g0 + h) * 256 + 64 * i + 64].reshape(16, 4).astype(np.float64)
+                            for j in range(4):      # the square is exact in f64: one rounding, as an FMA has
+                                lanes[w, hw] = (x[:, j] * x[:, j] + lanes[w, hw]).astype(np.float32)
+    v = lanes.reshape(warps, 32)
+    for o in (16, 8, 4, 2, 1):
+        v = v + v[:, np.arange(32) ^ o]
+    tot = v[0, 0]
+    for w in range(1, warps):
+        tot = np.float32(tot + v[w, 0])
+    return tot
+
+
+@pytest.mark.parametrize("k", [512, 3072, 8192, 8448, 12288, 16384, 17408])
+def test_rms_mod_takes_the_row_sum_in_one_order(be, k):
+    """The sum of squares decides the last bit of every element, and of the quantised values behind it: its order is part of the
+    result, whatever the number of warps a row is given."""
+    m = 40
+    u = rnd((m, k), seed=k)
+    mod = np.concatenate([np.ones(k, np.float32), np.zeros(k, np.float32)])
+    out = torch.empty((m, k), dtype=torch.float32, device="cuda")
+    be.rmsMod(dev(u), out, dev(mod), m, k, 0, k, EPS)
+    be.status_poll()
+    want = np.empty_like(u)
+    for r in range(m):
+        ms = np.float32(_rms_sum_of_squares(u[r]) / np.float32(k)) + np.float32(EPS)
+        want[r] = u[r] * np.float32(1.0 / np.sqrt(np.float64(ms)))
+    assert np.array_equal(out.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("count", [1, 2, 3, 4])
 @pytest.mark.parametrize("m,n,k", [(2048, 3072, 512), (2500, 2064, 256), (300, 512, 256)])
