@@ -240,41 +240,49 @@ int launch_cfg(tpb_handle_t h, cudaStream_t st, const GemmParams &p, const int8_
     return launch_cfg_p<BN, OUT, 0>(h, st, p, q, w8, b_unsigned);
 }
 
-// Which tile takes a problem: the one whose waves of tiles cost least.  A persistent CTA (or CTA pair) walks whole
-// tiles, so a launch takes ceil(tiles / SMs) rounds of k / 128 K blocks each, plus what does not overlap (launch,
-// pipeline fill, the last epilogue).  Measured per round and K block of 128 at k = 12288, and the rest at k = 3072 (us):
-//   128 x 64    0.295 + 3.0    (bound by shared-memory traffic: A is staged for 64 columns only)
-//   128 x 128   0.315 + 4.0
-//   128 x 192   0.365 + 4.3
-//   128 x 256   0.46  + 5.0
-//   256 x 256   0.41  + 5.5    on an SM pair
-// (256 x 192 on a pair took 0.39 a round: 0.95 of the 256-wide round for 0.75 of the work, never the best.)  E.g. m 1111,
-// n 3072, k 12288: 216 tiles of 128 x 128 are two rounds, 60 us; 144 of 128 x 192 are one, 34.5 us.  m 777, n 2048, k 4096:
-// two rounds of 128 x 64 28 us, one of 128 x 128 15 us.  m 2048, n 3072, k 12288: 96 pair tiles on 74 pairs 77 us,
-// 256 of 128 x 192 65 us.  The pair keeps a problem unless another tile is 4 % better: under the power cap, which a long
-// GEMM meets, its fewer bytes staged per product count for more than the bursts above show.
+// Which tile takes a problem: the one whose waves of tiles cost least.  A persistent CTA (or CTA pair) walks whole tiles, ceil(tiles /
+// SMs) rounds of them, with the epilogue of one tile beside the K blocks of the next: launch and pipeline fill, the first round's K blocks,
+// for every further round its K blocks or the epilogue, whichever takes longer, and the last epilogue.  Fitted to 241 shapes (m 130 ..
+// 4608, n 1024 .. 12288, k 256 .. 12288) times five tiles times three epilogues, rms error 6-8 % (us: fixed, per K block of 128, epilogue to
+// f32 / to bf16 / gated residual):
+//   128 x 64    1.9   0.295   1.3  1.0   2.5   (bound by shared-memory traffic: A is staged for 64 columns only)
+//   128 x 128   1.7   0.307   2.4  1.8   5.4
+//   128 x 192   1.9   0.312   3.9  2.7   8.1
+//   128 x 256   1.7   0.395   4.9  3.9  10.6
+//   256 x 256   2.0   0.338   5.3  4.5   9.3   on an SM pair
+// The choice is within 0.5 % of the best tile on average.  E.g. m 1111, n 3072, k 12288: 216 tiles of 128 x 128 are two rounds, 60 us; 144 of
+// 128 x 192 are one, 35 us.  m 777, n 2048, k 4096: two rounds of 128 x 64 23 us, one of 128 x 128 14.7.  m 2048, n 3072, k 12288: 96 pair tiles
+// on 74 pairs 69 us, 176 of 128 x 192 64 us.  m 3000, n 1536, k 1024: 72 pair tiles 10.7 us, two rounds of 128 x 128 9.8 (with the epilogue left out
+// of the rounds the pair looked cheaper).  The pair keeps a problem unless another tile is 8 % better (gated: 4 %): under the power cap,
+// which a long GEMM meets, its fewer bytes staged per product count for more than the bursts above show.
 enum Tile { S64, S128, S192, S256, P256 };
-double tile_us(int sms, Tile t, int64_t m, int64_t n, int64_t k, int count) {
-    static const struct { int bm, bn, sms; double per_block, fixed; } kCost[] = {
-        {128, 64, 1, 0.295, 3.0}, {128, 128, 1, 0.315, 4.0}, {128, 192, 1, 0.365, 4.3}, {128, 256, 1, 0.46, 5.0}, {256, 256, 2, 0.41, 5.5}};
+enum Epilogue { EPI_F32, EPI_BF16, EPI_GATED };
+double tile_us(int sms, Tile t, Epilogue epi, int64_t m, int64_t n, int64_t k, int count) {
+    static const struct { int bm, bn, sms; double fixed, per_block, epilogue[3]; } kCost[] = {
+        {128, 64, 1, 1.9, 0.295, {1.3, 1.0, 2.5}}, {128, 128, 1, 1.7, 0.307, {2.4, 1.8, 5.4}}, {128, 192, 1, 1.9, 0.312, {3.9, 2.7, 8.1}},
+        {128, 256, 1, 1.7, 0.395, {4.9, 3.9, 10.6}}, {256, 256, 2, 2.0, 0.338, {5.3, 4.5, 9.3}}};
     const auto &c = kCost[t];
     const int64_t tiles = (m + c.bm - 1) / c.bm * ((n + c.bn - 1) / c.bn) * count;
     const int64_t slots = sms / c.sms > 0 ? sms / c.sms : 1;
-    return (double)((tiles + slots - 1) / slots) * (double)(k / BK) * c.per_block + c.fixed;
+    const double blocks = (double)(k / BK) * c.per_block, e = c.epilogue[epi];
+    return c.fixed + blocks + (double)((tiles + slots - 1) / slots - 1) * (blocks > e ? blocks : e) + e;
 }
-Tile pick_tile(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double *us = nullptr) {
+Tile pick_tile(tpb_handle_t h, Epilogue epi, int64_t m, int64_t n, int64_t k, double *us = nullptr) {
+    // A gated residual larger than half of L2 or so: its reads and writes bound the launch, and the pair with its eight epilogue warps
+    // has most of them in flight (4608 x 3072, k 3072: pair 43.6 us, 128 x 192 52.7; 3000 x 8192, k 512: 63.7 against 69-93).
+    if (epi == EPI_GATED && m * n >= 14000000 && !h->opt_gemm_one_cta) return P256;
     Tile best = S64;
     double t_best = 0.0;
     for (int t = S64; t <= P256; t++) {
         if (t == P256 && h->opt_gemm_one_cta) break;
-        double v = tile_us(h->sm_count, (Tile)t, m, n, k, 1);
-        if (t == P256) v *= 0.96;
+        const double raw = tile_us(h->sm_count, (Tile)t, epi, m, n, k, 1);
+        const double v = t == P256 ? raw * (epi == EPI_GATED ? 0.96 : 0.92) : raw;
         if (t == S64 || v < t_best) {
             best = (Tile)t;
             t_best = v;
+            if (us) *us = raw;
         }
     }
-    if (us) *us = t_best;
     return best;
 }
 // The fused all-gather's epilogue also writes every other GPU's copy of the output, which the costs above do not hold:
@@ -344,7 +352,8 @@ int tpb_launch_gemm(tpb_handle_t h, cudaStream_t st, void *y, int y_dtype, int64
         w8 = buf;
     }
     // TPB_GEMM_ONE_CTA=1 keeps the one-CTA kernel for comparisons.
-    const Tile tile = n_peers > 0 || mc_y != nullptr ? pick_tile_peers(h, m, n) : pick_tile(h, m, n, k);
+    const Tile tile = n_peers > 0 || mc_y != nullptr ? pick_tile_peers(h, m, n)
+                                                            : pick_tile(h, gate ? EPI_GATED : y_dtype == TPB_BF16 ? EPI_BF16 : EPI_F32, m, n, k);
     if (tile == P256) return tpb_launch_gemm2(h, st, p, y_dtype, q, w8, false);
     switch (y_dtype) {
         case TPB_F32: return launch_out<OUT_F32>(h, st, p, q, w8, false, tile);
@@ -399,12 +408,13 @@ int tpb_launch_gemm_silu_pair(tpb_handle_t h, cudaStream_t st, void *y, int y_dt
 int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *const *y, int y_dtype, int64_t ldy,
                           const int8_t *q, const float *act_scale, const void *const *w, const float *const *w_scale,
                           int w_bits, int64_t m, int64_t n, int64_t k) {
+    const Epilogue epi = y_dtype == TPB_BF16 ? EPI_BF16 : EPI_F32;
     double one_us = 0.0;
-    pick_tile(h, m, n, k, &one_us);
+    pick_tile(h, epi, m, n, k, &one_us);
     // A reservation that covers one int4 weight only is enough for small problems, as it was when they always ran one by one.
     const bool small = (m + 255) / 256 * ((n + 255) / 256) < h->sm_count / 2;
     const bool scratch_for_one = w_bits == 4 && small && h->w4_scratch_bytes < (size_t)count * (size_t)n * (size_t)k;
-    if (h->opt_gemm_one_cta || scratch_for_one || 0.96 * tile_us(h->sm_count, P256, m, n, k, count) > count * one_us) {
+    if (h->opt_gemm_one_cta || scratch_for_one || 0.96 * tile_us(h->sm_count, P256, epi, m, n, k, count) > count * one_us) {
         for (int g = 0; g < count; g++) {
             const int rc = tpb_launch_gemm(h, st, y[g], y_dtype, ldy, q, act_scale, nullptr, w[g], w_bits, w_scale[g], m, n, k,
                                            nullptr, 0, nullptr, nullptr);

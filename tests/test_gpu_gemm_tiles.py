@@ -1,5 +1,5 @@
-"""The int8 GEMM picks one of five tiles by a cost per round of tiles; these shapes reach each of them (on 148 SMs) with
-row and column counts that are not multiples of the tile, and the group of several weights on both of its routes.  The int32
+"""The int8 GEMM picks one of five tiles by the cost of its rounds of tiles; these shapes reach each of them (on 148 SMs) with
+row and column counts that are not multiples of the tile, and the group of several weights.  The int32
 accumulators are exact; f32 and bf16 outputs are the two products of the contract, rounded once each."""
 import numpy as np
 import pytest
@@ -19,13 +19,18 @@ def be():
     b.close()
 
 
-SHAPES = [
-    (130, 1040, 512),      # 128 x 64
-    (777, 2032, 1024),     # 128 x 128
-    (1111, 3056, 512),     # 128 x 192, one round
-    (2000, 3072, 768),     # 128 x 192, two rounds
-    (890, 5360, 1024),     # 128 x 256
-    (2300, 2032, 1024),    # 256 x 256 on an SM pair
+SHAPES = [                  # the tile of the f32 output / of the gated residual
+    (130, 1040, 512),       # 128 x 64
+    (777, 2032, 1024),      # 128 x 128 / 128 x 64
+    (1111, 3056, 512),      # 128 x 64 (bf16: 128 x 192)
+    (2000, 3072, 768),      # 128 x 128 / 128 x 64, two rounds and more
+    (890, 5360, 1024),      # 128 x 128 / 128 x 64
+    (2300, 2032, 1024),     # 128 x 128 / 256 x 256
+    (700, 4080, 1024),      # 128 x 192 / 128 x 64
+    (890, 5360, 2048),      # 128 x 256 / 128 x 128
+    (2300, 2032, 2048),     # 256 x 256 on an SM pair
+    (396, 4880, 1536),      # gated: 128 x 192
+    (1025, 3648, 3072),     # 128 x 256, gated too
 ]
 
 
