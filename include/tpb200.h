@@ -153,7 +153,8 @@ int tpb_convrot_gemm_silu_pair(tpb_handle_t h, tpb_stream_t stream, void *y, int
  * persistent kernel, so its pipeline fills and drains once instead of count times (4608 x 3072 x 3072, four
  * weights: 4 x 36 us -> 131 us).  y, w and w_scale are host arrays of `count` device pointers (1 <= count <= 4).
  * For w_bits = 4 the reservation (tpb_convrot_w4_reserve) must cover all weights: count * n x k elements.
- * Problems too small for the two-CTA kernel run as `count` ordinary launches. */
+ * Where the two-CTA kernel fits the weights badly (two weights over a few tokens with short K, say) they run as
+ * `count` ordinary launches, with the same results. */
 int tpb_convrot_gemm_group(tpb_handle_t h, tpb_stream_t stream, int count, void *const *y, int y_dtype, int64_t ldy,
                            const int8_t *q, const float *act_scale, const int32_t *act_sum, const void *const *w,
                            const float *const *w_scale, int w_bits, int64_t m, int64_t n, int64_t k);

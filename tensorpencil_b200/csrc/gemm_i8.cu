@@ -403,8 +403,8 @@ int tpb_launch_gemm_silu_pair(tpb_handle_t h, cudaStream_t st, void *y, int y_dt
 // Up to four weights of one shape times the same activations in one launch of the two-CTA kernel (the q, k, v and
 // gate projections of a DiT block): their tiles follow one another in its persistent loop, so the pipeline fills
 // and drains once instead of once per weight, and the last round is shared by all of them.  One by one where a tile of
-// the one-CTA kernel fits a single weight so much better that it pays (m 256, n = k = 3072: 41 us one by one, 18 together;
-// m 1111, k 12288: 4 x 35 one by one, 141 together).
+// the one-CTA kernel fits a single weight so much better that it pays: two weights of m 2048, n 12288, k 512 to bf16 46 us one by one,
+// 54 together, of m 256, n 3072, k 256 7.3 / 8.0; but four of m 256, n = k = 3072 41 / 17, four of m 1111, n 3072, k 12288 143 / 141.
 int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *const *y, int y_dtype, int64_t ldy,
                           const int8_t *q, const float *act_scale, const void *const *w, const float *const *w_scale,
                           int w_bits, int64_t m, int64_t n, int64_t k) {
@@ -414,7 +414,9 @@ int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *cons
     // A reservation that covers one int4 weight only is enough for small problems, as it was when they always ran one by one.
     const bool small = (m + 255) / 256 * ((n + 255) / 256) < h->sm_count / 2;
     const bool scratch_for_one = w_bits == 4 && small && h->w4_scratch_bytes < (size_t)count * (size_t)n * (size_t)k;
-    if (h->opt_gemm_one_cta || scratch_for_one || 0.96 * tile_us(h->sm_count, P256, epi, m, n, k, count) > count * one_us) {
+    // the pair's bonus where it holds (pick_tile): in a launch long enough to meet the power cap
+    const double together_us = (small ? 1.0 : 0.96) * tile_us(h->sm_count, P256, epi, m, n, k, count);
+    if (h->opt_gemm_one_cta || scratch_for_one || together_us > count * one_us) {
         for (int g = 0; g < count; g++) {
             const int rc = tpb_launch_gemm(h, st, y[g], y_dtype, ldy, q, act_scale, nullptr, w[g], w_bits, w_scale[g], m, n, k,
                                            nullptr, 0, nullptr, nullptr);

@@ -302,7 +302,7 @@ def test_rms_mod_takes_the_row_sum_in_one_order(be, k):
 def test_gemm_group_is_bit_identical_to_separate_gemms(be, bits, count, m, n, k):
     """Several weights of one shape on the same prepped activations in one launch (the q, k, v and gate
     projections of a block): every output equals the separate GEMM's, bit for bit, f32 and bf16 -- on a
-    problem the two-CTA kernel takes, one with ragged edges, and one small enough for the one-by-one path."""
+    problem the two-CTA kernel takes, one with ragged edges, and one so small that two weights run one by one."""
     from tensorpencil_b200 import synth
     cs = [synth.convrot_linear(m, n, k, bits, seed=71 + 3 * g + m) for g in range(count)]
     key = "w_i8" if bits == 8 else "w_packed"

@@ -79,9 +79,51 @@ def test_group_of_small_weights_matches_the_single_calls(be, m, n, k):
         assert all(torch.equal(a, b) for a, b in zip(got, want)), dt
 
 
+def _kernels_in(fn):
+    """Number of kernel launches of fn, from the nodes of a captured graph."""
+    import ctypes as C
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g, stream=stream):
+            fn()
+        n = C.c_size_t(0)
+        rt = C.CDLL("libcudart.so.12")
+        rt.cudaGraphGetNodes.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_size_t)]
+        assert rt.cudaGraphGetNodes(g.raw_cuda_graph(), None, C.byref(n)) == 0
+    torch.cuda.synchronize()
+    return n.value
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("count,m,n,k,together", [(2, 16, 9728, 3072, False), (2, 300, 512, 256, False), (2, 256, 3072, 256, False),
+                                                  (4, 300, 512, 256, True), (4, 256, 3072, 3072, True), (2, 2048, 3072, 512, True)])
+def test_group_route_and_results(be, bits, count, m, n, k, together):
+    """Both routes of the group with several weights, int4 with scratch reserved for all of them: which one it is shows in the number
+    of launches (int4 adds one per weight to widen it), and every output equals the single call's."""
+    rng = np.random.default_rng(m + n + bits)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    be.reserveW4(count * n, k)
+    be._prep(dev(rng.standard_normal((m, k)).astype(np.float32)), m, k, bits)
+    if bits == 8:
+        ws = [dev(rng.integers(-128, 128, size=(n, k), dtype=np.int8)) for _ in range(count)]
+    else:
+        ws = [dev(rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)) for _ in range(count)]
+    sc = [dev(rng.uniform(0.5, 1.5, n).astype(np.float32)) for _ in range(count)]
+    want = [torch.empty((m, n), device="cuda") for _ in ws]
+    for y, w, s in zip(want, ws, sc):
+        be._gemm(y, w, s, n, bits)
+    got = [torch.full((m, n), 3.0, device="cuda") for _ in ws]
+    be.gemmGroup(got, ws, sc, n, bits)
+    be.status_poll()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    launches = _kernels_in(lambda: be.gemmGroup(got, ws, sc, n, bits))
+    assert launches == (1 if together else count) + (count if bits == 4 else 0)
+
+
 def test_group_of_small_int4_weights_needs_scratch_for_one_only():
-    """Small groups used to run one by one, so a reservation for a single weight served them: it still does (larger groups need
-    all their weights reserved, as the header says)."""
+    """Small groups once always ran one by one, so a reservation for a single weight served them: it still does, and they run one by
+    one then (larger groups need all their weights reserved, as the header says)."""
     from tensorpencil_b200 import _lib
     from tensorpencil_b200.backend import Backend
     m, n, k = 200, 512, 512
