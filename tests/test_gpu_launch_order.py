@@ -66,6 +66,71 @@ def test_linear_sees_the_activations_of_its_own_iteration(be, bits):
     assert all(torch.equal(y, ref[i % 3]) for i, y in enumerate(ys))
 
 
+def _same_without_synchronising(be, call, xs, iters=60):
+    """call(x) -> result, over inputs that change every iteration: back to back, and with a synchronisation after every call."""
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        ref = []
+        for x in xs:
+            ref.append(call(x))
+            torch.cuda.synchronize()
+        got = [call(xs[i % len(xs)]) for i in range(iters)]
+        torch.cuda.synchronize()
+    be.status_poll()
+    assert not torch.equal(ref[0], ref[1])
+    assert all(torch.equal(y, ref[i % len(xs)]) for i, y in enumerate(got))
+
+
+@pytest.mark.parametrize("n,k", [(14336, 4096), (1024, 1024), (512, 768)])
+def test_f32_gemv_sees_the_activations_of_its_own_iteration(be, n, k):
+    from tensorpencil_b200 import harness
+    w = harness.rotating_q8_weights(n, k, 1, be.device)[0]
+    src = [torch.randn(1, k, device="cuda") * (1 + i) for i in range(3)]
+    x = torch.empty(1, k, device="cuda")
+
+    def call(s):
+        x.zero_()
+        be.gatedAdd(x, s, torch.ones_like(x), k, k, 0)      # the kernel in front writes x, and lets its successor start early
+        y = torch.empty(1, n, device="cuda")
+        be.opGemvQuant("q8_0", y, x, w, 1.0, n, k)
+        return y
+
+    _same_without_synchronising(be, call, src)
+
+
+@pytest.mark.parametrize("kernel", ["warp", "mma"])
+@pytest.mark.parametrize("m", [1, 4, 8])
+@pytest.mark.parametrize("fmt,n,k", [("q4_k", 5120, 5120), ("q6_k", 1024, 17408), ("iq4_nl", 2048, 2304)])
+def test_gguf_gemv_sees_the_activations_of_its_own_iteration(be, fmt, n, k, m, kernel, monkeypatch):
+    from tensorpencil_b200 import synth
+    monkeypatch.setenv("TPB_GEMVK_KERNEL", kernel)
+    w = torch.from_numpy(synth.gguf_weights(fmt, n, k, seed=n + m)).cuda()
+
+    def call(x):
+        y = torch.empty(m, n, device="cuda")
+        be.opGemvQuantizeX(x, m * k)
+        be.opGemvQuantQ8N(fmt, y, w, 1.0, n, k, m, 0, m)
+        return y
+
+    _same_without_synchronising(be, call, [torch.randn(m, k, device="cuda") * (1 + i) for i in range(3)])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("seq,heads,kv_heads", [(700, 12, 4), (77, 3, 1)])
+def test_attention_sees_the_tokens_of_its_own_iteration(be, dtype, seq, heads, kv_heads):
+    """The prepare pass writes into the buffers that the attention kernel in front of it still reads."""
+    qn, kn = torch.rand(128, device="cuda") + 0.5, torch.rand(128, device="cuda") + 0.5
+    ang = torch.rand(seq, 64, device="cuda") * 6.28
+    cos, sin = ang.cos(), ang.sin()
+    xs = [[torch.randn(seq, h * 128, device="cuda").to(dtype) * (1 + i) for h in (heads, kv_heads, kv_heads)] for i in range(3)]
+
+    def call(qkv):
+        return be.attention(*qkv, qn, kn, cos, sin, heads, kv_heads)
+
+    _same_without_synchronising(be, call, xs)
+
+
 class _WrittenWeights:
     """Q8_0 weights whose bytes a kernel writes on the stream just before they are used.  All bytes lie in 0x20 .. 0x2f: as pairs they
     are finite f16 scales, as quants 32 .. 47, and as words normal f32 numbers, so x = 0 + 1 * source writes them exactly."""
