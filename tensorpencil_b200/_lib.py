@@ -9,10 +9,12 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import os
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libtpb200.so")
-CALL_PATH = os.path.join(_HERE, "lib", "_tpbcall.so")
+# built for one interpreter: the suffix names its ABI, so that another one does not load it
+CALL_PATH = os.path.join(_HERE, "lib", "_tpbcall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 TPB_OK = 0
 TPB_ERR_INVALID_ARG = -1
@@ -112,19 +114,42 @@ def load() -> C.CDLL:
     return lib
 
 
+class CtypesCalls:
+    """The functions of csrc/pycall.c through ctypes, for an interpreter that the extension is not built for."""
+
+    def __init__(self, lib: C.CDLL):
+        self._lib = lib
+
+    def __getattr__(self, name):
+        fn = getattr(self._lib, name)
+        setattr(self, name, fn)
+        return fn
+
+    def q8_0_linear(self, h, stream, y, x, m, w, scale, rows, cols, xq):
+        rc = self._lib.tpb_q8_1_quantize(h, stream, x, m * cols, xq)
+        for r0 in range(0, m, 8):
+            if rc != TPB_OK:
+                break
+            rc = self._lib.tpb_q8_0_gemv_q8n(h, stream, y + 4 * r0 * rows, w, scale, rows, cols, xq, min(8, m - r0), r0, m)
+        return rc
+
+
 _calls = None
 
 
 def load_calls():
     """The same functions, for the calls made once per weight, without ctypes' argument conversion (csrc/pycall.c):
-    pointers and integers as Python integers (None = NULL), scales as floats."""
+    pointers and integers as Python integers (None = NULL), scales as floats.  Where the extension is not built for this
+    interpreter the calls are made through ctypes, with the same arguments and results."""
     global _calls
     if _calls is None:
-        load()
-        if not os.path.exists(CALL_PATH):
-            raise RuntimeError(f"{CALL_PATH} is missing: build it with `python -m tensorpencil_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader("_tpbcall", CALL_PATH)
-        spec = importlib.util.spec_from_loader("_tpbcall", loader)
-        _calls = importlib.util.module_from_spec(spec)
-        loader.exec_module(_calls)
+        lib = load()
+        if os.path.exists(CALL_PATH):
+            loader = importlib.machinery.ExtensionFileLoader("_tpbcall", CALL_PATH)
+            spec = importlib.util.spec_from_loader("_tpbcall", loader)
+            calls = importlib.util.module_from_spec(spec)
+            loader.exec_module(calls)
+        else:
+            calls = CtypesCalls(lib)
+        _calls = calls
     return _calls

@@ -15,13 +15,15 @@ import subprocess
 import sys
 import sysconfig
 
+from ._lib import CALL_PATH
+
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OUT_DIR = os.path.join(PKG, "lib")
 LIB = os.path.join(OUT_DIR, "libtpb200.so")
 OBJ_DIR = os.path.join(OUT_DIR, "obj")
-PYCALL = os.path.join(OUT_DIR, "_tpbcall.so")   # CPython entry to the hot calls (csrc/pycall.c)
+PYCALL_SRC = os.path.join(CSRC, "pycall.c")
 
 SOURCES = ["api.cu", "prep.cu", "prep_fused.cu", "gemm_i8.cu", "gemm2_i8.cu", "gemm_w4.cu", "qgemv.cu", "qgemv_mma.cu", "qgemv_k.cu", "qgemv_kmma.cu", "offload.cu", "peer.cu", "attn.cu"]
 
@@ -46,6 +48,19 @@ def _stale(target: str, deps) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def build_pycall(out: str, lib_dir: str) -> bool:
+    """The CPython entry to the hot calls (csrc/pycall.c) for the running interpreter, linked to lib_dir/libtpb200.so, by the compiler that
+    nvcc drives.  Without Python's headers it is left out, and the calls go through ctypes (_lib.load_calls)."""
+    inc = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(inc, "Python.h")):
+        sys.stderr.write(f"{inc}/Python.h not found: {os.path.basename(out)} is not built, calls go through ctypes\n")
+        return False
+    subprocess.run([_nvcc(), "-O2", "-Xcompiler", "-fPIC,-Wall", "-shared", "-cudart", "none", "-I", inc,
+                    "-I", os.path.join(ROOT, "include"), PYCALL_SRC, "-o", out, "-L", lib_dir, "-Xlinker", "-l:libtpb200.so",
+                    "-Xlinker", "-rpath,$ORIGIN"], check=True)
+    return True
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -77,11 +92,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-cudart", "static",
                                                      "-Xlinker", "--no-undefined"]
         subprocess.run(cmd, check=True, env=env)
-    src = os.path.join(CSRC, "pycall.c")
-    if force or _stale(PYCALL, [src, headers[0]]):
-        subprocess.run(["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"],
-                        "-I", os.path.join(ROOT, "include"), src, "-o", PYCALL, "-L", OUT_DIR, "-l:libtpb200.so",
-                        "-Wl,-rpath,$ORIGIN"], check=True)
+    if force or _stale(CALL_PATH, [PYCALL_SRC, headers[0]]):
+        build_pycall(CALL_PATH, OUT_DIR)
     return LIB
 
 
