@@ -414,6 +414,12 @@ int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *cons
     // A reservation that covers one int4 weight only is enough for small problems, as it was when they always ran one by one.
     const bool small = (m + 255) / 256 * ((n + 255) / 256) < h->sm_count / 2;
     const bool scratch_for_one = w_bits == 4 && small && h->w4_scratch_bytes < (size_t)count * (size_t)n * (size_t)k;
+    // A larger one needs every weight reserved, whichever route is the faster.
+    int8_t *all_weights = nullptr;
+    if (w_bits == 4 && !small && !h->opt_gemm_one_cta) {
+        const int rc = tpb_w4_scratch(h, (int64_t)count * n, k, &all_weights);
+        if (rc != TPB_OK) return rc;
+    }
     // the pair's bonus where it holds (pick_tile): in a launch long enough to meet the power cap
     const double together_us = (small ? 1.0 : 0.96) * tile_us(h->sm_count, P256, epi, m, n, k, count);
     if (h->opt_gemm_one_cta || scratch_for_one || together_us > count * one_us) {

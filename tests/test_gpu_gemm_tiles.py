@@ -97,7 +97,8 @@ def _kernels_in(fn):
 
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("count,m,n,k,together", [(2, 16, 9728, 3072, False), (2, 300, 512, 256, False), (2, 256, 3072, 256, False),
-                                                  (4, 300, 512, 256, True), (4, 256, 3072, 3072, True), (2, 2048, 3072, 512, True)])
+                                                  (4, 300, 512, 256, True), (4, 256, 3072, 3072, True), (2, 2048, 3072, 512, True),
+                                                  (4, 1, 16, 256, True), (3, 33, 48, 512, True)])
 def test_group_route_and_results(be, bits, count, m, n, k, together):
     """Both routes of the group with several weights, int4 with scratch reserved for all of them: which one it is shows in the number
     of launches (int4 adds one per weight to widen it), and every output equals the single call's."""
@@ -147,4 +148,28 @@ def test_group_of_small_int4_weights_needs_scratch_for_one_only():
     b._prep(dev(rng.standard_normal((4096, k)).astype(np.float32)), 4096, k, 4)
     with pytest.raises(_lib.TpbError):
         b.gemmGroup([torch.zeros((4096, 4608), device="cuda") for _ in range(2)], wide, ws2, 4608, 4)
+    b.close()
+
+
+@pytest.mark.parametrize("n", [3072, 12288])
+def test_large_int4_group_needs_scratch_for_all_weights_on_both_routes(n):
+    """A group of more than a round of pair tiles has always needed every weight reserved; that one by one would do with one does
+    not depend on which of the two is faster (n 12288: one by one)."""
+    from tensorpencil_b200 import _lib
+    from tensorpencil_b200.backend import Backend
+    m, k = 2048, 512
+    b = Backend(0)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    rng = np.random.default_rng(n)
+    ws = [dev(rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)) for _ in range(2)]
+    sc = [torch.ones(n, device="cuda") for _ in ws]
+    ys = [torch.zeros((m, n), device="cuda") for _ in ws]
+    b._prep(dev(rng.standard_normal((m, k)).astype(np.float32)), m, k, 4)
+    b.reserveW4(n, k)
+    reserved, b._w4_reserved = b._w4_reserved, 1 << 40          # the mirror asks for no more
+    with pytest.raises(_lib.TpbError):
+        b.gemmGroup(ys, ws, sc, n, 4)
+    b._w4_reserved = reserved
+    b.gemmGroup(ys, ws, sc, n, 4)
+    b.status_poll()
     b.close()
