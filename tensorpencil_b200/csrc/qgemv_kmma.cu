@@ -25,7 +25,7 @@
 // launch costs nearly the same whatever the number of activation rows is: q4_k 17408 x 5120 17.0 us at M = 1, 18.1 at 8 (floor 7.8),
 // where the dp4a kernel takes 12.5 and 32.2.  us at M = 8, dp4a / here: 5120 x 17408 q4_k 56 / 27, q5_k 65 / 31, q6_k 87 / 43;
 // 17408 x 5120 q5_k 35 / 23, q6_k 45 / 29; 32000 x 4096 q4_k 52 / 23; 4096 x 14336 q4_0 39 / 18, iq4_nl 50 / 24.  The dispatch rule
-// stands at tpb_gguf_gemv_q8n.
+// is mma_wins in qgemv_k.cu.
 //
 // Rows of a stage are `pitch` bytes apart with pitch = 48 mod 128: the eight rows of a fragment load (8 x 16 or
 // 4 x 32 bytes at a time) then fall on distinct banks.

@@ -65,7 +65,9 @@ int tpb_fail(tpb_handle_t h, int code, const char *fmt, ...);
 // Launch with programmatic stream serialisation: the grid may start while the previous
 // kernel in the stream is still draining.  Every kernel launched this way executes
 // griddepcontrol.wait before it reads or writes global memory, which also keeps the
-// ordering transitive along the stream.  Data that another kernel of the stream may have written
+// ordering transitive along the stream -- but for the weights of the GEMVs on quantised activations, which
+// those kernels begin to stream ahead of the wait (the header says what orders them; the quantiser in front of
+// them, which does, lets its successor start only after its own wait).  Data that another kernel of the stream may have written
 // (activations, scales, modulation vectors, residuals) is loaded with __ldcg, never __ldg: a load
 // through the read-only path counts as invariant for the compiler, which may move it above
 // griddepcontrol.wait, where it reads what the previous kernel has not written yet.  __ldg is for
