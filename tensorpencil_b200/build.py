@@ -25,7 +25,7 @@ LIB = os.path.join(OUT_DIR, "libtpb200.so")
 OBJ_DIR = os.path.join(OUT_DIR, "obj")
 PYCALL_SRC = os.path.join(CSRC, "pycall.c")
 
-SOURCES = ["api.cu", "prep.cu", "prep_fused.cu", "gemm_i8.cu", "gemm2_i8.cu", "gemm_w4.cu", "qgemv.cu", "qgemv_mma.cu", "qgemv_k.cu", "qgemv_kmma.cu", "offload.cu", "peer.cu", "attn.cu"]
+SOURCES = ["api.cu", "prep.cu", "prep_fused.cu", "gemm_i8.cu", "gemm2_i8.cu", "gemm_splitk.cu", "gemm_w4.cu", "qgemv.cu", "qgemv_mma.cu", "qgemv_k.cu", "qgemv_kmma.cu", "offload.cu", "peer.cu", "attn.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -70,6 +70,7 @@ int tpb_create(tpb_handle_t *out, int device_ordinal) {
         if (e == cudaSuccess && (qres != cudaDriverEntryPointSuccess || !h->encode_tiled))
             e = cudaErrorUnknown;
     }
+    if (e == cudaSuccess) tpb_gemm_splitk_init(h);
     cudaSetDevice(prev);
     if (e != cudaSuccess) {
         if (h->d_status) cudaFree(h->d_status);

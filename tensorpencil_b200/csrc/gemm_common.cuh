@@ -37,6 +37,7 @@ struct TileCfg {
     static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;
 };
 
+constexpr int kMaxSplit = 8;  // CTAs that share a tile's K (gemm_splitk.cu): the portable cluster size
 constexpr int kMaxPeers = 7;  // world size <= 8
 
 struct GemmParams {

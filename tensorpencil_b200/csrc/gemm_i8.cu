@@ -28,6 +28,8 @@ int tpb_launch_gemm2_silu_pair(tpb_handle_t h, cudaStream_t st, const tpb_gemm::
                                const int8_t *q, const void *w_gate, const void *w_up);
 int tpb_launch_gemm2(tpb_handle_t h, cudaStream_t st, const tpb_gemm::GemmParams &p, int y_dtype,
                      const int8_t *q, const void *w8, bool b_unsigned);
+int tpb_launch_gemm_splitk(tpb_handle_t h, cudaStream_t st, const tpb_gemm::GemmParams &p, int y_dtype, const int8_t *q, const void *w8,
+                           int bn, int split);
 int tpb_launch_gemm_w4(tpb_handle_t h, cudaStream_t st, const tpb_gemm::GemmParams &p, int y_dtype,
                         const int8_t *q, const void *w4);
 
@@ -285,6 +287,35 @@ Tile pick_tile(tpb_handle_t h, Epilogue epi, int64_t m, int64_t n, int64_t k, do
     }
     return best;
 }
+// Whether the CTAs of a cluster share a tile's K (gemm_splitk.cu), and how: for problems whose tiles leave SMs idle and whose K is a long chain.
+// One round of clusters only, as many as the device holds at once; the cost of a choice is linear in the K blocks of a part, the rows whose
+// parts are sent and added, and the bytes that all SMs load (us, fitted to 128 shapes x 18 choices, rms error 6-8 %).  us, one
+// chain / split: m 16, n 1024, k 12288 29.5 / 8.4; m 64, n 3072, k 6144 16.8 / 9.0; m 256, n 1024, k 3072 10.1 / 6.1; m 256, n = k = 3072 10.5 / 8.3;
+// m 297, n 3072, k 12288 30.6 / 21.4; m 1, n 16, k 1024 4.3 / 3.0.  Over 384 shapes and epilogues with m 16 .. 1111 the choice is 1.28 x as fast as
+// one chain on average and nowhere more than 2 % slower.  Several rounds of clusters lost everywhere (m 512, n 5008, k 3072: 13.9 / 25).
+struct Split { int bn = 0, parts = 1; };
+Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta_us) {
+    static const struct { int bn; double fixed, per_block, rows, rows_part, load; } kCost[] = {
+        {64, 2.84, 0.260, 1.51, -2.13, 0.112}, {128, 3.10, 0.345, 2.08, -2.10, 0.080}, {192, 3.49, 0.352, 2.85, -1.90, 0.265}};
+    Split best;
+    double t_best = 0.96 * one_cta_us;
+    const int64_t blocks = k / BK;
+    const double rows = (double)(m < BM ? m : BM) / BM;
+    for (const auto &c : kCost) {
+        const int64_t tiles = (m + BM - 1) / BM * ((n + c.bn - 1) / c.bn);
+        for (int parts = 2; parts <= kMaxSplit && parts <= blocks; parts++) {
+            if (tiles > h->max_clusters[parts]) break;
+            const double b = (double)((blocks + parts - 1) / parts);
+            const double us = c.fixed + c.per_block * b + c.rows * rows + c.rows_part * rows / parts + c.load * b * (double)(tiles * parts) / h->sm_count;
+            if (us < t_best) {
+                best.bn = c.bn;
+                best.parts = parts;
+                t_best = us;
+            }
+        }
+    }
+    return best;
+}
 // The fused all-gather's epilogue also writes every other GPU's copy of the output, which the costs above do not hold:
 // there the widest tile that still gives every SM (pair) work.
 Tile pick_tile_peers(tpb_handle_t h, int64_t m, int64_t n) {
@@ -352,8 +383,15 @@ int tpb_launch_gemm(tpb_handle_t h, cudaStream_t st, void *y, int y_dtype, int64
         w8 = buf;
     }
     // TPB_GEMM_ONE_CTA=1 keeps the one-CTA kernel for comparisons.
-    const Tile tile = n_peers > 0 || mc_y != nullptr ? pick_tile_peers(h, m, n)
-                                                            : pick_tile(h, gate ? EPI_GATED : y_dtype == TPB_BF16 ? EPI_BF16 : EPI_F32, m, n, k);
+    Tile tile;
+    if (n_peers > 0 || mc_y != nullptr) {
+        tile = pick_tile_peers(h, m, n);
+    } else {
+        double us = 0.0;
+        tile = pick_tile(h, gate ? EPI_GATED : y_dtype == TPB_BF16 ? EPI_BF16 : EPI_F32, m, n, k, &us);
+        const Split split = pick_split(h, m, n, k, us);
+        if (split.parts > 1) return tpb_launch_gemm_splitk(h, st, p, y_dtype, q, w8, split.bn, split.parts);
+    }
     if (tile == P256) return tpb_launch_gemm2(h, st, p, y_dtype, q, w8, false);
     switch (y_dtype) {
         case TPB_F32: return launch_out<OUT_F32>(h, st, p, q, w8, false, tile);

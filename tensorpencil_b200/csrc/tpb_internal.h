@@ -32,6 +32,7 @@ struct tpb_handle_s {
     int sm_count = 0;
     int smem_optin = 0;
     uint32_t *d_status = nullptr;   // device status word written by bounded waits
+    int max_clusters[9] = {0};      // clusters of 2 .. 8 CTAs of the split-K GEMM that the device holds at once; 0: not used
     // cuTensorMapEncodeTiled, resolved through the runtime so the library has no
     // link-time dependency on libcuda (it must load on a host without a driver).
     void *encode_tiled = nullptr;
@@ -76,20 +77,28 @@ int tpb_fail(tpb_handle_t h, int code, const char *fmt, ...);
 // writes is never declared `const __restrict__`: that qualifier lets the compiler pick the
 // read-only path by itself.
 template <typename... KArgs, typename... Args>
-static inline cudaError_t tpb_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                         cudaStream_t st, Args... args) {
+static inline cudaError_t tpb_launch_pdl_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                                 cudaStream_t st, int cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     static const bool no_pdl = getenv("TPB_NO_PDL") != nullptr;
     attr[0].val.programmaticStreamSerializationAllowed = no_pdl ? 0 : 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;   // cluster <= 1: none, or the one that the kernel declares
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t tpb_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                         cudaStream_t st, Args... args) {
+    return tpb_launch_pdl_cluster(kern, grid, block, smem, st, 1, args...);
 }
 
 #ifdef __CUDACC__
@@ -133,6 +142,7 @@ static inline cudaError_t tpb_set_max_smem_once(tpb_handle_t h, Kern kern, int b
 
 static inline bool tpb_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+void tpb_gemm_splitk_init(tpb_handle_t h);   // sizes of the split-K GEMM's clusters; h's device is current
 // Kernel launchers (one per .cu file).  All return a tpb_status.
 int tpb_launch_prep(tpb_handle_t h, cudaStream_t st, const void *x, int x_dtype, int64_t m,
                     int64_t k, int bits, int8_t *q, float *act_scale, int32_t *act_sum);
