@@ -58,7 +58,8 @@ struct PrepParams {
     float *act_scale;
     int32_t *act_sum;
     int m, k, n_groups;
-    float maxq;
+    float maxq, rcp_maxq;
+    int ahead;            // rows between a CTA's row and the one whose input it asks into L2; 0 = none
 };
 
 // 16 packed int4 bytes -> 32 int8 bytes (element 2j in the low nibble, src/core/dtype.zig:146-149)
@@ -236,7 +237,18 @@ __device__ __forceinline__ float sigmoid_fast(float x) {
     return r;
 }
 
+// max(a, |b|, |c|) in one instruction; like fmaxf, a NaN operand is ignored
+__device__ __forceinline__ float max_abs3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(fabsf(b)), "f"(fabsf(c)));
+    return d;
+}
+
 constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23: adding it leaves rint(x) in the low mantissa bits
+
+__device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 
 // UPW = units (pairs of groups) per half-warp (compile time, sizes the register file use).
 // ONE_WARP: the row fits one warp (k <= 1024): every warp of the CTA takes its own row and
@@ -262,6 +274,11 @@ convrot_prep_kernel(const PrepParams P) {
     const T *brow = static_cast<const T *>(P.b) + (size_t)row * k;
     tpb_grid_dep_launch();
     tpb_grid_dep_wait();
+    if (P.ahead != 0 && warp == 0 && lane == 0 && row + P.ahead < P.m) {
+        const size_t off = (size_t)P.ahead * k;
+        l2_prefetch(arow + off, (uint32_t)k * (uint32_t)sizeof(T));
+        if (OP == OP_SILU_MUL || OP == OP_SIGMOID_MUL) l2_prefetch(brow + off, (uint32_t)k * (uint32_t)sizeof(T));
+    }
 
     f2 v[UPW][4][4];
     float sumsq = 0.0f;
@@ -405,25 +422,29 @@ convrot_prep_kernel(const PrepParams P) {
             for (int j = 0; j < 4; j++) {
                 float lo, hi;
                 unpack2(v[p][i][j], lo, hi);
-                amax = fmaxf(amax, fmaxf(fabsf(lo), fabsf(hi)));
+                amax = max_abs3(amax, lo, hi);
             }
     }
 
-    // Row absmax: warp butterfly, then across the CTA's warps.
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    // Row absmax, never negative and never a NaN: its bits compare like the integers they are, in one instruction per warp.
+    amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
     if (!ONE_WARP) {
         if (lane == 0) s_max[warp] = amax;
         __syncthreads();
-        amax = s_max[0];
-        for (int w = 1; w < n_warps; w++) amax = fmaxf(amax, s_max[w]);
+        amax = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < n_warps ? __float_as_uint(s_max[lane & (kMaxWarpsWide - 1)]) : 0u));
     }
 
     // The values above are 16x the rotated ones; /16 is exact, so the absmax of
     // the rotated row is amax/16 and v/16/s == v/(16 s) as correctly rounded floats.
-    const float s = fmaxf(__fdiv_rn(amax * 0.0625f, P.maxq), 1e-12f);
+    // The quotient by maxq (127 or 7) is corrected once with its exact remainder (Markstein 1990), which rounds it correctly for
+    // every dividend that leaves a scale above 1e-12; an infinite absmax stays one.
+    const float a16 = amax * 0.0625f;
+    const float q0 = a16 * P.rcp_maxq;
+    const float quot = a16 > 3.402823466e38f ? a16 : __fmaf_rn(__fmaf_rn(-q0, P.maxq, a16), P.rcp_maxq, q0);
+    const float s = fmaxf(quot, 1e-12f);
     const float s16 = s * 16.0f;
-    const float rcp = __frcp_rn(s16);
+    float rcp;   // within 1 ulp, and a normal number: s16 is in [1.6e-11, 2^125.2]
+    asm("rcp.approx.f32 %0, %1;" : "=f"(rcp) : "f"(s16));
     if (warp == 0 && lane == 0) P.act_scale[row] = s;
     const f2 rcp2 = pack2(rcp, rcp);
     const f2 magic2 = pack2(kRoundMagic, kRoundMagic);
@@ -434,8 +455,8 @@ convrot_prep_kernel(const PrepParams P) {
         const int g0 = 2 * ((2 * warp + hw) + p * 2 * n_warps);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            // Fast path: v*rcp is within 2e-5 of the IEEE quotient for |q| <= 128, so
-            // unless it sits within 1e-4 of a half-integer, rounding it to nearest gives
+            // Fast path: v*rcp is within 1.9e-5 of the IEEE quotient for |q| <= 127 (2^-23 of it from rcp, 2^-18 from the quotient's own
+            // rounding), so unless it sits within 2.5e-5 of a half-integer, rounding it to nearest gives
             // round-half-away(v / s) exactly.  y = rint(v*rcp) + magic in one FMA; the
             // distance of v*rcp from that integer in a second one.
             f2 y[4];
@@ -446,10 +467,10 @@ convrot_prep_kernel(const PrepParams P) {
                 const f2 neg_int = sub2(magic2, y[j]);  // -(rint(v*rcp)), exact
                 float dl, dh;
                 unpack2(fma2(v[p][i][j], rcp2, neg_int), dl, dh);
-                tie = fmaxf(tie, fmaxf(fabsf(dl), fabsf(dh)));
+                tie = max_abs3(tie, dl, dh);
             }
             uint32_t yb[2][4];
-            if (tie > 0.4999f) {
+            if (tie > 0.499975f) {
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     float lo, hi;
@@ -479,17 +500,15 @@ convrot_prep_kernel(const PrepParams P) {
         }
     }
     if (P.act_sum != nullptr) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) isum += __shfl_xor_sync(0xffffffffu, isum, o);
+        isum = __reduce_add_sync(0xffffffffu, isum);
         if (ONE_WARP) {
             if (lane == 0) P.act_sum[row] = isum;
         } else {
             if (lane == 0) s_sum[warp] = isum;
             __syncthreads();
-            if (threadIdx.x == 0) {
-                int t = 0;
-                for (int w = 0; w < n_warps; w++) t += s_sum[w];
-                P.act_sum[row] = t;
+            if (warp == 0) {
+                isum = __reduce_add_sync(0xffffffffu, lane < n_warps ? s_sum[lane & (kMaxWarpsWide - 1)] : 0);
+                if (lane == 0) P.act_sum[row] = isum;
             }
         }
     }
@@ -511,9 +530,20 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
     P.k = (int)k;
     P.n_groups = n_groups;
     P.maxq = bits == 4 ? 7.0f : 127.0f;
+    P.rcp_maxq = 1.0f / P.maxq;
+    // Inputs asked into L2 half a wave of rows ahead of the CTA that reads them: with 32 warps on an SM, loads in flight alone do not cover
+    // HBM's latency, and a request of one thread for a whole row costs no registers.  For 16-bit inputs and RMS norm (which waits for its row twice)
+    // from five waves on; f32 rows are long enough in flight, two of them more so, and a short launch only gets a second stream beside its first.
+    // us without / a wave ahead / half of one: bf16 4608 x 12288 plain 50.8 / 49.9 / 49.5, SiLU gate 85.7 / 75.9 / 74.6, RMS 99.8 / 95.0 / 93.5; f32
+    // RMS 4608 x 12288 110.7 / 105.1 / 102.3; but f32 plain 4608 x 3072 16.3 / 18.8 / 17.3, SiLU gate 113 / 121 / 118, bf16 1111 x 12288 plain 15.0 / 15.3 / 15.1.
+    auto set_ahead = [&](int rows_per_sm) {
+        const int64_t wave = (int64_t)rows_per_sm * h->sm_count;
+        P.ahead = (sizeof(T) == 2 || OP == OP_RMS_MOD) && m >= 5 * wave ? (int)(wave / 2) : 0;
+    };
     cudaError_t err = cudaSuccess;
     if (n_units <= 2) {
         const dim3 grid((unsigned)((m + kRowsPerCta - 1) / kRowsPerCta)), block(kRowsPerCta * 32);
+        set_ahead(32);
         const size_t smem = ACT_ONLY ? 0 : (size_t)kRowsPerCta * 2 * kTilePairs * sizeof(f2);
         err = tpb_launch_pdl(convrot_prep_kernel<T, 1, OP, ACT_ONLY, true>, grid, block, smem, st, P);
     } else {
@@ -530,6 +560,7 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
         const int upw = (n_units + 2 * max_warps - 1) / (2 * max_warps);  // 1..4 for k <= 32768
         const int warps = (n_units + 2 * upw - 1) / (2 * upw);
         const dim3 grid((unsigned)m), block(warps * 32);
+        set_ahead(32 / warps);
         const size_t smem = ACT_ONLY ? 0 : (size_t)warps * 2 * kTilePairs * sizeof(f2);
 #define TPB_PREP_CASE(UU)                                                                               \
     case UU: {                                                                                          \
