@@ -19,6 +19,8 @@
 // warp, and y = acc * scale.
 #include <cuda_fp16.h>
 
+#include <cmath>
+
 
 #include "qgemv_common.cuh"
 
@@ -32,6 +34,10 @@ constexpr int kChunkBlocks = 2 * kPairsPerChunk;   // 64 blocks
 constexpr int kChunkBytes = kChunkBlocks * kBlockBytes;  // 2176 per row (multiple of 16)
 constexpr int kActPairBytes = 80;  // a block pair's 64 activation bytes + 16 pad: 16-byte reads at lane stride 80 hit distinct banks
 __host__ __device__ constexpr int stage_bytes(int rows_per_group) { return rows_per_group * kChunkBytes; }
+
+// Warps per CTA of the dp4a kernel, at most: twenty (96 registers a thread) for one and two activation rows, where more warps still hide more
+// latency and rows are dealt out to them in pairs; with more activation rows the arithmetic of sixteen fills the time.
+__host__ __device__ constexpr int q8n_max_warps(int m, int r) { return r != 2 ? 8 : m <= 2 ? 20 : 16; }
 
 struct GemvParams {
     float *y;
@@ -47,7 +53,7 @@ struct GemvParams {
 // ACT_SMEM: activations staged in shared memory.  Every warp of the grid owns a
 // contiguous, nearly equal range of weight rows.
 template <int M, int R, bool ACT_SMEM>
-__global__ void __launch_bounds__(R == 2 ? 512 : 256, 1)
+__global__ void __launch_bounds__(32 * q8n_max_warps(M, R), 1)
 q8_0_gemv_q8n_kernel(const GemvParams p, const int stages) {
     constexpr int kRows = R;
     constexpr int kStageBytes = stage_bytes(R);
@@ -82,8 +88,9 @@ q8_0_gemv_q8n_kernel(const GemvParams p, const int stages) {
     const int cpr = (nblk + kChunkBlocks - 1) / kChunkBlocks;  // chunks per row
     const int gw = blockIdx.x * n_warps + warp;
     const int GW = gridDim.x * n_warps;
-    const int my_r0 = (int)((long long)p.rows * gw / GW);        // this warp's rows: [my_r0, my_r1)
-    const int my_r1 = (int)((long long)p.rows * (gw + 1) / GW);
+    int my_r0 = (int)((long long)p.rows * gw / GW);              // this warp's rows: [my_r0, my_r1)
+    int my_r1 = (int)((long long)p.rows * (gw + 1) / GW);
+    if (q8n_max_warps(M, R) > 16) warp_row_pairs(p.rows, gw, GW, my_r0, my_r1);
     const int my_rg = (my_r1 - my_r0 + kRows - 1) / kRows;       // groups of up to R rows
     const int total = my_rg * cpr;
 
@@ -336,7 +343,8 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
 // 3.6 us.  The rings fill after griddepcontrol.wait: this entry point has always seen a weight that the kernel in front of it wrote
 // (filled ahead of the wait the same launches took 14.7, 21.4, 13.2 and 2.8 us).
 constexpr int kF32PairBytes = 272;
-__global__ void __launch_bounds__(512, 1)
+constexpr int kF32Warps = 20;
+__global__ void __launch_bounds__(32 * kF32Warps, 1)
 q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ w, float scale, int rows, int cols, int stages,
                           uint32_t *status) {
     constexpr int R = 2;
@@ -364,8 +372,8 @@ q8_0_gemv_f32_ring_kernel(float *y, const float *x, const uint8_t *__restrict__ 
     const int cpr = (nblk + kChunkBlocks - 1) / kChunkBlocks;  // chunks per row
     const int gw = blockIdx.x * n_warps + warp;
     const int GW = gridDim.x * n_warps;
-    const int my_r0 = (int)((long long)rows * gw / GW);
-    const int my_r1 = (int)((long long)rows * (gw + 1) / GW);
+    int my_r0, my_r1;
+    warp_row_pairs(rows, gw, GW, my_r0, my_r1);
     const int total = (my_r1 - my_r0 + R - 1) / R * cpr;
 
     int is_c = 0, is_row = my_r0, is_st = 0;
@@ -501,16 +509,21 @@ static GemvOverride gemv_override() {
 }
 
 // Warps per CTA and stages per warp of the dp4a kernel for one rows-per-stage choice (stage = its bytes); 0 warps:
-// the activations leave no room.  Every warp owns a contiguous range of whole rows, so the slowest warp
-// carries ceil(rows / warps_total) rows.  Among the counts that fit (with >= 2 stages and the activations in
-// shared memory) take the one with the best balance; ties go to more warps.  E.g. 5120 rows on 148 SMs:
+// the activations leave no room.  The slowest warp carries ceil(rows / warps_total) rows.  Among the counts that fit (with >= 2 stages and
+// the activations in shared memory) take the one with the best balance; ties go to more warps.  E.g. 5120 rows on 148 SMs:
 // 16 warps -> 2.16 rows per warp (3 vs 2, 72 %), 12 warps -> 2.88 (96 %).
+// Kernels that may have more than sixteen warps deal rows out in pairs, one a step (warp_row_pairs).  What counts then is the share of the
+// warps' steps that is work -- a third of it, as the last steps of the slowest warps run on an SM that is half empty and so faster -- how evenly the warps
+// fill the SM's four schedulers, and a little how many there are.  us at M = 1, at most sixteen warps with ranges cut at any row / so: 5120 x 5120
+// 7.9 / 6.6 (twelve warps with two steps / eighteen with one), 17408 x 5120 17.8 / 17.2, 14336 x 4096 12.3 / 11.9, 5120 x 17408 20.3 / 17.8, 20000 x 2304 18.8 / 13.1,
+// 32000 x 4096 23.3 / 23.3 (on 20 warps 24.3); the f32 kernel 5120 x 5120 10.7 / 9.4, 14336 x 4096 16.5 / 14.8, 17408 x 5120 23.6 / 21.3, 5120 x 17408 27.2 / 21.7.
+// Over 31 shapes of each 1.04 x on average, the worst 0.97.
 static void dp4a_plan(tpb_handle_t h, size_t act, int64_t rows, int stage, int max_warps, int max_stages, int *warps, int *stages) {
     const size_t limit = (size_t)h->smem_optin - 1024;
     *warps = 0;
     *stages = 0;
     double best_eff = -1.0;
-    for (int w = max_warps; w >= max_warps / 2; w--) {
+    for (int w = max_warps; w >= (max_warps < 16 ? max_warps / 2 : 8); w--) {
         int s_fit = 0;
         for (int s = max_stages; s >= 2; s--)
             if (act + (size_t)w * s * stage + (size_t)w * s * 8 + 64 <= limit) {
@@ -519,8 +532,14 @@ static void dp4a_plan(tpb_handle_t h, size_t act, int64_t rows, int stage, int m
             }
         if (s_fit == 0) continue;
         const double per_warp = (double)rows / ((double)h->sm_count * w);
-        const double eff = per_warp >= 1.0 ? per_warp / (double)(long long)(per_warp + 0.999999) : per_warp;
-        if (eff > best_eff + 0.02) {
+        double eff = per_warp >= 1.0 ? per_warp / (double)(long long)(per_warp + 0.999999) : per_warp;
+        double margin = 0.02;
+        if (max_warps > 16 && per_warp > 2.0) {
+            const double n = per_warp * 0.5, idle = (double)(long long)(n + 0.999999) - n;
+            eff = n / (n + 0.35 * idle) * ((double)w / (double)(4 * ((w + 3) / 4))) * pow((double)w / max_warps, 0.1);
+            margin = 0.0;
+        }
+        if (eff > best_eff + margin) {
             best_eff = eff;
             *warps = w;
             *stages = s_fit;
@@ -602,7 +621,7 @@ int launch_q8n(tpb_handle_t h, cudaStream_t st, const GemvParams &p) {
     // hiding).  When the activations leave too little shared memory for that, 8 warps with
     // 4 rows each (activations are re-read from shared memory once per R rows).
     if (gemv_override().r != 4) {
-        const int rc = launch_q8n_cfg<M, 2>(h, st, p, 16);
+        const int rc = launch_q8n_cfg<M, 2>(h, st, p, q8n_max_warps(M, 2));
         if (rc != TPB_ERR_STATE) return rc;  // TPB_ERR_STATE: did not fit, try the wider grouping
     }
     return launch_q8n_cfg<M, 4>(h, st, p, 8);
@@ -649,7 +668,7 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
             // the dp4a kernel at its best: fourteen warps with two two-row stages each fit beside the activations
             // (with fewer its time jumps: K = 14336 from the sixth activation row on, K = 28672 from the third)
             int warps = 0, stages = 0;
-            dp4a_plan(h, act_bytes, rows, stage_bytes(2), 16, q8n_stages(h, rows, cols), &warps, &stages);
+            dp4a_plan(h, act_bytes, rows, stage_bytes(2), q8n_max_warps(ng, 2), q8n_stages(h, rows, cols), &warps, &stages);
             const bool roomy = warps != 0 && act_bytes + 14 * 2 * (size_t)stage_bytes(2) + 14 * 2 * 8 + 64 <=
                                                  (size_t)h->smem_optin - 1024;
             // share of its row slots that hold a row: rows come to a warp two at a time
@@ -711,7 +730,7 @@ int tpb_launch_q8_0_gemv_f32(tpb_handle_t h, cudaStream_t st, float *y, const fl
     if (cols % 256 == 0 && cols >= (rows < 64 ? 2048 : 1024)) {
         const size_t act = (size_t)(cols / 64) * kF32PairBytes;
         int warps = 0, stages = 0;
-        dp4a_plan(h, act, rows, stage_bytes(2), 16, 2, &warps, &stages);
+        dp4a_plan(h, act, rows, stage_bytes(2), kF32Warps, 2, &warps, &stages);
         if (warps != 0) {
             int rgrid = (int)((rows + 2 * warps - 1) / (2 * warps));
             if (rgrid > h->sm_count) rgrid = h->sm_count;
