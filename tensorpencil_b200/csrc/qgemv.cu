@@ -339,8 +339,8 @@ q8_0_gemv_f32_kernel(float *__restrict__ y, const float *__restrict__ x, const u
 //
 // What bounds it: 2.25 instructions a weight for that, the two multiply-adds and their operands from shared memory (8 KB of
 // activations per two rows of 2048), against 62.4 MB of weights at 14336 x 4096 (9.5 us at 6.55 TB/s): 72.6 us with the
-// 16-bit global loads of the kernel above -> 16.2 us = 3.9 TB/s; 17408 x 5120 113 -> 23.5 us, 4096 x 14336 87 -> 14.6 us, 1024 x 4096 9.7 ->
-// 3.6 us.  The rings fill after griddepcontrol.wait: this entry point has always seen a weight that the kernel in front of it wrote
+// 16-bit global loads of the kernel above -> 14.8 us = 4.2 TB/s; 17408 x 5120 113 -> 21.3 us, 4096 x 14336 87 -> 14.5 us, 1024 x 4096 9.7 ->
+// 3.6 us (rows cut at any row to at most sixteen warps: 16.5 and 23.6).  The rings fill after griddepcontrol.wait: this entry point has always seen a weight that the kernel in front of it wrote
 // (filled ahead of the wait the same launches took 14.7, 21.4, 13.2 and 2.8 us).
 constexpr int kF32PairBytes = 272;
 constexpr int kF32Warps = 20;
@@ -653,8 +653,8 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
     // (qgemv_mma.cu) costs the same whatever M is, but 0-4 us more than the dp4a kernel's single row (more where its
     // per-warp K slices are padded, K = 4096: 4 block pairs in MMAs built for 6, and where it needs two passes
     // over K).  Measured on ten decode shapes, M = 1 .. 8 (us, dp4a / mma): 17408 x 5120  17.6 19.1 21.0 23.8 /
-    // 19.2-20.0;  5120 x 17408  21.1 22.9 25.4 / 19.9-21.4 (few long rows: the dp4a kernel's warps get 2.9 rows
-    // for two-row stages);  32000 x 4096  22.6 22.7 24.8 26.7 29.9 / 27.1-28.7;  4096 x 14336  11.6 12.7 13.7 15.1
+    // 19.2-20.0;  5120 x 17408  21.1 22.9 25.4 / 19.9-21.4 (few long rows: 2.9 of
+    // them a warp for two-row stages; eighteen warps with one step each take 17.8 and 18.8 for one and two activation rows);  32000 x 4096  22.6 22.7 24.8 26.7 29.9 / 27.1-28.7;  4096 x 14336  11.6 12.7 13.7 15.1
     // 16.9 26.7 / 15.3-16.2;  8192 x 28672  41.0 42.2 69.6 / 49.8-53.0;  28672 x 8192  41.4 42.4 43.6 47.9 /
     // 41.4-44.9.  The rule below follows that table.  TPB_GEMV_KERNEL=dp4a / mma forces one.
     {

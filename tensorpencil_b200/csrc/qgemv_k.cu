@@ -48,6 +48,10 @@ template <> struct Fmt<FMT_IQ4_NL> { static constexpr int kUnitBytes = 36; };
 template <> struct Fmt<FMT_Q4_K> { static constexpr int kUnitBytes = 36; };   // 144 / 4
 template <> struct Fmt<FMT_Q5_K> { static constexpr int kUnitBytes = 44; };   // 176 / 4
 
+// For one and two activation rows, weight rows may be dealt out to the warps in pairs, one a step (kq_plan); with more of them a step with a
+// single row costs much less than one with two, and how evenly the rows divide is what counts.
+__host__ __device__ constexpr bool kq_pairs(int m) { return m <= 2; }
+
 struct KGemvParams {
     float *y;
     const uint8_t *w;
@@ -56,6 +60,7 @@ struct KGemvParams {
     float scale;
     int rows, cols, nblk;  // nblk = cols / 32
     size_t row_bytes;
+    bool pairs;            // dp4a kernels at M <= 2: rows are dealt out in pairs (kq_plan)
     uint32_t chunk_pitch;  // ring kernel: bytes between the rows of a stage
     uint32_t *status;
 };
@@ -239,8 +244,9 @@ kquant_gemv_q8n_kernel(const KGemvParams p, const int stages) {
     const int cpr = (n_units + kUnitsPerChunk - 1) / kUnitsPerChunk;  // chunks per row
     const int gw = blockIdx.x * n_warps + warp;
     const int GW = gridDim.x * n_warps;
-    const int my_r0 = (int)((long long)p.rows * gw / GW);
-    const int my_r1 = (int)((long long)p.rows * (gw + 1) / GW);
+    int my_r0 = (int)((long long)p.rows * gw / GW);
+    int my_r1 = (int)((long long)p.rows * (gw + 1) / GW);
+    if (kq_pairs(M) && p.pairs) warp_row_pairs(p.rows, gw, GW, my_r0, my_r1);
     const int my_rg = (my_r1 - my_r0 + R - 1) / R;
     const int total = my_rg * cpr;
 
@@ -616,8 +622,9 @@ q6k_gemv_q8n_kernel(const KGemvParams p, const int stages) {
     const int cpr = (n_sb + kQ6ChunkSb - 1) / kQ6ChunkSb;
     const int gw = blockIdx.x * n_warps + warp;
     const int GW = gridDim.x * n_warps;
-    const int my_r0 = (int)((long long)p.rows * gw / GW);
-    const int my_r1 = (int)((long long)p.rows * (gw + 1) / GW);
+    int my_r0 = (int)((long long)p.rows * gw / GW);
+    int my_r1 = (int)((long long)p.rows * (gw + 1) / GW);
+    if (kq_pairs(M) && p.pairs) warp_row_pairs(p.rows, gw, GW, my_r0, my_r1);
     const int my_rg = (my_r1 - my_r0 + R - 1) / R;
     const int total = my_rg * cpr;
 
@@ -862,10 +869,16 @@ static size_t kq_stage_bytes(int fmt, int ng, int64_t cols) {
 }
 // Warps per CTA: every warp owns a contiguous range of whole rows; among the counts that fit with >= 2 stages take the one whose
 // ranges divide most evenly (ties: more warps).
-static void kq_plan(tpb_handle_t h, size_t act, size_t stage, int64_t rows, int max_stages, int *warps, int *stages) {
+// With more than one step a warp, rows may be dealt out in pairs (pairs != null): the cost of a count is then its average number of steps and, as the last
+// ones run on an SM that is half empty, a third of what the slowest warp has above it, over how evenly the warps fill the four schedulers.  Ranges cut
+// at any row cost half a step a row; pairs are taken where they come out 2 % lower.  us at M = 1, cut / in pairs: 14336 x 4096 q4_k 9.8 (14 warps of 6.92 rows) /
+// 9.1 (16 of 3.03 pairs), q5_k 11.8 / 10.8, q6_k 13.8 / 12.9, iq4_nl 16.5 / 15.4; 5120 x 5120 q4_k 7.2 / 6.8, q6_k 11.7 / 10.7; 13500 x 6144 q4_k 19.9 / 10.8;
+// but 7000 x 3072 (2.96 rows, 1.48 pairs) iq4_nl 9.0 / 9.9, 3072 x 3072 q5_k 4.8 / 5.0.
+static void kq_plan(tpb_handle_t h, size_t act, size_t stage, int64_t rows, int max_stages, int *warps, int *stages, bool *pairs) {
     const size_t limit = (size_t)h->smem_optin - 1024;
     *warps = *stages = 0;
-    double best_eff = -1.0;
+    double best_eff = -1.0, cut_cost = 0.0, pair_cost = 0.0;
+    int pair_warps = 0, pair_stages = 0;
     for (int w = 16; w >= 4; w--) {
         int s_fit = 0;
         for (int s = max_stages; s >= 2; s--)
@@ -874,13 +887,27 @@ static void kq_plan(tpb_handle_t h, size_t act, size_t stage, int64_t rows, int 
                 break;
             }
         if (s_fit == 0) continue;
-        const double per_warp = (double)rows / ((double)h->sm_count * w);
-        const double eff = per_warp >= 1.0 ? per_warp / (double)(long long)(per_warp + 0.999999) : per_warp;
+        const double per_warp = (double)rows / ((double)h->sm_count * w), most = (double)(long long)(per_warp + 0.999999);
+        const double eff = per_warp >= 1.0 ? per_warp / most : per_warp;
         if (eff > best_eff + 0.02) {
             best_eff = eff;
             *warps = w;
             *stages = s_fit;
+            cut_cost = 0.5 * most;
         }
+        const double steps = 0.5 * per_warp, top = (double)(long long)(steps + 0.999999);
+        const double cost = (steps + 0.35 * (top - steps)) * (double)(4 * ((w + 3) / 4)) / w;
+        if (pair_warps == 0 || cost < pair_cost) {
+            pair_cost = cost;
+            pair_warps = w;
+            pair_stages = s_fit;
+        }
+    }
+    if (pairs == nullptr) return;
+    *pairs = rows > 2ll * 16 * h->sm_count && pair_warps != 0 && pair_cost < 0.98 * cut_cost;
+    if (*pairs) {
+        *warps = pair_warps;
+        *stages = pair_stages;
     }
 }
 
@@ -909,7 +936,7 @@ static bool mma_wins(tpb_handle_t h, int fmt, int64_t rows, int64_t cols, int m)
     if (m < 3 || weights < 5000000) return false;
     int warps = 0, stages = 0;
     const int max_stages = fmt == TPB_GGUF_Q6_K ? 4 : kq_max_stages(rows, tpb_gguf_row_bytes(fmt, cols));
-    kq_plan(h, kq_act_bytes(fmt, m, cols), kq_stage_bytes(fmt, m, cols), rows, max_stages, &warps, &stages);
+    kq_plan(h, kq_act_bytes(fmt, m, cols), kq_stage_bytes(fmt, m, cols), rows, max_stages, &warps, &stages, nullptr);
     if (warps <= 5 && weights >= 20000000) return true;
     const double per_cta = (double)rows / h->sm_count > 4.0 ? (double)rows / h->sm_count : 4.0;
     const double fill = per_cta / (16.0 * (double)((long long)(per_cta / 16.0 + 0.999999)));
@@ -958,7 +985,8 @@ int launch_q6k_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     constexpr int kStage = R * kQ6RowStage;
     const size_t act = kq_act_bytes(TPB_GGUF_Q6_K, M, p.cols);
     int warps = 0, stages = 0;
-    kq_plan(h, act, kStage, p.rows, 4, &warps, &stages);
+    bool pairs = false;
+    kq_plan(h, act, kStage, p.rows, 4, &warps, &stages, kq_pairs(M) ? &pairs : nullptr);
     if (stages == 0)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "gguf_gemv: %d activation rows of %d columns do not fit shared memory",
                         M, p.cols);
@@ -969,7 +997,9 @@ int launch_q6k_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     auto kern = q6k_gemv_q8n_kernel<M, R>;
     static tpb_per_device_once smem_set;   // the size varies per call: opt in to the device maximum, once
     TPB_CUDA(h, tpb_set_max_smem_once(h, kern, h->smem_optin, smem_set));
-    TPB_CUDA(h, tpb_launch_pdl(kern, dim3(grid), dim3(warps * 32), smem, st, p, stages));
+    KGemvParams pp = p;
+    pp.pairs = pairs;
+    TPB_CUDA(h, tpb_launch_pdl(kern, dim3(grid), dim3(warps * 32), smem, st, pp, stages));
     return TPB_OK;
 }
 
@@ -993,7 +1023,8 @@ int launch_fmt_mu(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     constexpr int kStage = R * 32 * U * Fmt<FMT>::kUnitBytes;
     const size_t act = (size_t)M * (p.cols / 64) * kActPairBytes + (size_t)M * p.nblk * 8;
     int warps = 0, stages = 0;
-    kq_plan(h, act, kStage, p.rows, kq_max_stages(p.rows, p.row_bytes), &warps, &stages);
+    bool pairs = false;
+    kq_plan(h, act, kStage, p.rows, kq_max_stages(p.rows, p.row_bytes), &warps, &stages, kq_pairs(M) ? &pairs : nullptr);
     if (stages == 0)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "gguf_gemv: %d activation rows of %d columns do not fit shared memory",
                         M, p.cols);
@@ -1004,7 +1035,9 @@ int launch_fmt_mu(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     auto kern = kquant_gemv_q8n_kernel<FMT, M, R, U>;
     static tpb_per_device_once smem_set;   // the size varies per call: opt in to the device maximum, once
     TPB_CUDA(h, tpb_set_max_smem_once(h, kern, h->smem_optin, smem_set));
-    TPB_CUDA(h, tpb_launch_pdl(kern, dim3(grid), dim3(warps * 32), smem, st, p, stages));
+    KGemvParams pp = p;
+    pp.pairs = pairs;
+    TPB_CUDA(h, tpb_launch_pdl(kern, dim3(grid), dim3(warps * 32), smem, st, pp, stages));
     return TPB_OK;
 }
 
@@ -1144,6 +1177,7 @@ int tpb_gguf_gemv_q8n(tpb_handle_t h, tpb_stream_t stream, int fmt, float *y, co
                                  row_off + first, n_total);
     }
     KGemvParams p;
+    p.pairs = false;
     p.y = y;
     p.w = reinterpret_cast<const uint8_t *>(w);
     p.xd = reinterpret_cast<const float *>(xq) + (size_t)row_off * nblk;
