@@ -11,9 +11,9 @@
 //                store them, a warp to whole rows of the tile.
 // A tile's rows, as far as the problem has them, are split evenly over the cluster, so the last step has the whole cluster's SMs too.
 // What bounds it (cycle stamps, m 256, n = k = 3072 as 128 x 128 tiles on 48 pairs, 1.9 GHz): 1500 cycles until the first load is asked for,
-// 7200 for twelve K blocks (the first load's latency, then 600 a block: L2 to SM), 700 to stage and send the parts, 1300 until the peer's are there, 1700 for
-// sums and stores.  With four warps for the sums 1150 and 3350; with one barrier.cluster.sync at each end 500 and 1300 more; parts padded to 144
-// bytes a row instead of swizzled left no room for 192 columns.
+// 7200 for twelve K blocks (the first load's latency, then 600 a block: L2 to SM), and, with four warps for it, 1150 to stage and send the parts, 1350 until the
+// peer's are there, 3350 for sums and stores; eight warps took the launch from 9.5 to 9.0 us.  One barrier.cluster.sync at each end cost 500 and
+// 1300 more; parts padded to 144 bytes a row instead of swizzled left no room for 192 columns.
 // Every wait is bounded, and the cluster barrier at the end keeps a CTA's shared memory alive until all its copies have arrived.  No
 // load or copy here uses cluster multicast.
 #include "gemm_common.cuh"
