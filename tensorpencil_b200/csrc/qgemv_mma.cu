@@ -44,6 +44,12 @@
 // another consumer warp.  (Handing a stage back before the arithmetic, from registers, and letting
 // the last consumer warp add the partials were both measured: slower.)
 //
+// "Full" barriers are counted apart from the slots: stage j has slot j mod S and full barrier j mod F, F the smallest
+// multiple of the K segments that is at least S.  A wait names a phase by its parity, so it is only sound for a warp that has seen the
+// phase before it end, and a warp waits for the stages of its own segment alone.  With barriers counted like slots and five
+// slots for two segments, a warp could meet a barrier whose previous stage, the other segment's, was still on
+// its way (copies end in any order), take that phase for its own and multiply what lay in the slot.
+//
 // Rows in shared memory start 4 words apart modulo 32 banks, so the 8 rows x 4 words an A fragment
 // load touches fall in 32 different banks.
 //
@@ -68,6 +74,8 @@ constexpr int kThreadsMma = (kConsumers + kProducers) * 32;
 constexpr int kStageRows = 8;                  // weight rows per stage (rows 0..7 of the MMA's m side)
 constexpr int kActRows = 8;                    // activation rows = n of the MMA
 constexpr int kPartFloats = kStageRows * kActRows;
+constexpr int kMaxStages = 12;
+constexpr int kMaxBars = 32;                   // full and empty barriers: 16 + 12 at most
 
 struct MmaGemvParams {
     float *y;
@@ -82,6 +90,7 @@ struct MmaGemvParams {
     int grp_rows;      // rows one bulk copy brings in (1, 2, 4 or 8; > 1 only when a stage is whole rows)
     int grp_shift;     // extra bytes before every further copy's rows (keeps the 8 rows on distinct banks)
     int stages;        // ring depth
+    int full_bars;     // full barriers (full_bar_count)
     int rgbuf;         // row groups of partial sums kept
     int out_rg;        // K split: row groups of unscaled sums a CTA keeps for the final addition
     uint32_t *status;
@@ -93,6 +102,8 @@ struct MmaGemvParams {
 // cycles on the GPU -- four of them per stage made the producer warps the bottleneck of the kernel.)
 __host__ __device__ inline int pass_blk0(int nblk, int npass, int p) { return (nblk / 8) * p / npass * 8; }
 __host__ __device__ inline int seg_blk0(int pb0, int pb1, int nseg, int s) { return pb0 + ((pb1 - pb0) / 8) * s / nseg * 8; }
+// Full barriers of a ring of `stages` slots: no fewer, and each of them always of the same K segment.
+__host__ __device__ inline int full_bar_count(int stages, int nseg) { return (stages + nseg - 1) / nseg * nseg; }
 // pairs [lo, hi) of consumer `wi` (0 .. wps-1) inside a segment of `pairs` block pairs
 __host__ __device__ inline int warp_pair0(int pairs, int wps, int wi) { return pairs * wi / wps; }
 
@@ -132,7 +143,7 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int nblk = p.nblk;
-    const int S = p.stages;
+    const int S = p.stages, F = p.full_bars;
     const int stage_bytes = kStageRows * p.pitch + (kStageRows / p.grp_rows) * p.grp_shift;
     const size_t row_bytes = (size_t)nblk * kBlockBytes;
 
@@ -140,11 +151,11 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
     float *s_dx = reinterpret_cast<float *>(smem + (size_t)S * stage_bytes);       // [nblk][8 activation rows]
     float *s_part = s_dx + (size_t)kActRows * nblk;                                 // [rgbuf][kConsumers][8 weight rows x 8 activation rows]
     const uint32_t bars = smem_u32(s_part + (size_t)p.rgbuf * kConsumers * kPartFloats);
-    auto full_bar = [&](int s) { return bars + 8u * s; };
-    auto empty_bar = [&](int s) { return bars + 8u * (S + s); };
+    auto full_bar = [&](int f) { return bars + 8u * f; };
+    auto empty_bar = [&](int s) { return bars + 8u * (F + s); };
     // first block of every (pass, segment), plus one entry that closes the last segment of each pass:
     // s_seg[pass * (nseg + 1) + seg]; looked up instead of recomputed (integer divisions) per stage
-    int *s_seg = reinterpret_cast<int *>(s_part + (size_t)p.rgbuf * kConsumers * kPartFloats) + 2 * 2 * 16;
+    int *s_seg = reinterpret_cast<int *>(s_part + (size_t)p.rgbuf * kConsumers * kPartFloats) + 2 * kMaxBars;
     // K split: this CTA's passes are passes crank * npass .. of npass * KS over the whole row
     const int crank = KS > 1 ? (int)cluster_rank() : 0;
     const int npt = p.npass * KS;
@@ -157,10 +168,8 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
 
     const int wps = kConsumers / p.nseg;  // consumer warps per K segment
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S; s++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full_bar(s)), "r"(kProducers + 1));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty_bar(s)), "r"(wps));
-        }
+        for (int f = 0; f < F; f++) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full_bar(f)), "r"(kProducers + 1));
+        for (int s = 0; s < S; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty_bar(s)), "r"(wps));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -178,14 +187,14 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
     if (warp >= kConsumers) {
         // ---------------- producers (the first one also adds the partial sums) ----------------
         const int pw = warp - kConsumers;
-        // the stage the next issue() fills: (pass, row group, segment), ring slot, all advanced by one per call
-        int is_pass = 0, is_rg = 0, is_seg = 0, is_slot = 0;
+        // the stage the next issue() fills: (pass, row group, segment), ring slot, full barrier, all advanced by one per call
+        int is_pass = 0, is_rg = 0, is_seg = 0, is_slot = 0, is_bar = 0;
         auto issue = [&]() {  // whole warp: lane l starts copy number pw + 4 l of the next stage (a copy = grp_rows rows)
             const int row0 = r_begin + is_rg * kStageRows;
             const int nrow = min(kStageRows, r_end - row0);
             const int b0 = s_seg[is_pass * (p.nseg + 1) + is_seg], b1 = s_seg[is_pass * (p.nseg + 1) + is_seg + 1];
             const uint32_t bytes = (uint32_t)(b1 - b0) * kBlockBytes;   // per row
-            const uint32_t bar = full_bar(is_slot);
+            const uint32_t bar = full_bar(is_bar);
             const int cp = pw + kProducers * lane;                      // this lane's copy
             const int cp_row0 = cp * p.grp_rows;
             const int cp_rows = max(0, min(p.grp_rows, nrow - cp_row0));
@@ -202,6 +211,7 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
                 bulk_g2s(dst + (uint32_t)(cp_row0 * p.pitch + cp * p.grp_shift), src + (size_t)cp_row0 * row_bytes,
                          bytes * (uint32_t)cp_rows, bar);
             if (++is_slot == S) is_slot = 0;
+            if (++is_bar == F) is_bar = 0;
             if (++is_seg == p.nseg) {
                 is_seg = 0;
                 if (++is_rg == n_rg) {
@@ -253,7 +263,7 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
         };
         // weights are constants: the ring starts filling before the previous kernel has finished
         for (int i = 0; i < S && i < total; i++) {
-            if (pw == 0 && lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar(is_slot)) : "memory");
+            if (pw == 0 && lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full_bar(is_bar)) : "memory");
             issue();
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -266,7 +276,7 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
             ok = mbar_wait(empty_bar(w_slot), w_par, p.status, (7u << 24) | (uint32_t)w_slot);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
-            const uint32_t refill_bar = full_bar(is_slot);
+            const uint32_t refill_bar = full_bar(is_bar);
             if (j + S < total) {
                 // order the consumers' generic-proxy reads of the slot before the async-proxy refill
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -301,9 +311,9 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     bool ok = true;
-    // this warp's next stage: ring slot and phase (it takes every nseg-th stage), partial buffer
-    int c_slot = seg % S, c_pbuf = 0;
-    uint32_t c_par = (uint32_t)(seg / S) & 1u;
+    // this warp's next stage: ring slot, full barrier and phase (it takes every nseg-th stage), partial buffer
+    int c_slot = seg % S, c_bar = seg, c_pbuf = 0;
+    uint32_t c_par = 0;
   for (int pass = 0; pass < p.npass && ok; pass++) {
     const int sb0 = s_seg[pass * (p.nseg + 1) + seg], sb1 = s_seg[pass * (p.nseg + 1) + seg + 1];
     const int seg_pairs = (sb1 - sb0) / 2;
@@ -375,7 +385,7 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
     const uint32_t dx_u32 = smem_u32(s_dx + (size_t)(sb0 + 2 * pp0) * kActRows + 2 * t);
 
     for (int rg = 0; rg < n_rg && ok; rg++) {
-        ok = mbar_wait(full_bar(c_slot), c_par, p.status, (8u << 24) | (uint32_t)c_slot);
+        ok = mbar_wait(full_bar(c_bar), c_par, p.status, (8u << 24) | (uint32_t)c_slot);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         const uint32_t wl = ring_u32 + (uint32_t)(c_slot * stage_bytes);
@@ -422,8 +432,10 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(empty_bar(c_slot)) : "memory");
         c_slot += p.nseg;
-        while (c_slot >= S) {
-            c_slot -= S;
+        while (c_slot >= S) c_slot -= S;
+        c_bar += p.nseg;
+        if (c_bar >= F) {
+            c_bar -= F;
             c_par ^= 1u;
         }
         if (++c_pbuf == p.rgbuf) c_pbuf = 0;
@@ -505,8 +517,8 @@ MmaPlan plan_mma_ks(tpb_handle_t h, int nblk, int ks, size_t extra) {
                 pitch = pitch_w * 4;
             }
             const size_t stage = (size_t)kStageRows * pitch + (size_t)(kStageRows / grp_rows) * grp_shift;
-            const size_t fixed = (size_t)kActRows * nblk * 4 + 64 + 2 * 8 * 16 + 4 * 8 * 17;   // + the segment table
-            for (int stages = 12; stages >= 3; stages--) {
+            const size_t fixed = (size_t)kActRows * nblk * 4 + 64 + 8 * kMaxBars + 4 * 8 * 17;   // + the segment table
+            for (int stages = kMaxStages; stages >= 3; stages--) {
                 const int rgbuf = (stages - 1 + nseg - 1) / nseg + 1;
                 const size_t smem = stages * stage + fixed + (size_t)rgbuf * kConsumers * kPartFloats * 4;
                 if (smem > limit) continue;
@@ -603,6 +615,7 @@ int tpb_launch_q8_0_gemv_mma(tpb_handle_t h, cudaStream_t st, float *y, const vo
     p.grp_rows = pl.grp_rows;
     p.grp_shift = pl.grp_shift;
     p.stages = pl.stages;
+    p.full_bars = full_bar_count(pl.stages, pl.nseg);
     p.rgbuf = pl.rgbuf;
     p.out_rg = pl.out_rg;
     p.status = h->d_status;
