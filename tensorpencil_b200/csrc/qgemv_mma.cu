@@ -23,7 +23,8 @@
 // across a cluster of two CTAs instead: both stream the same rows (twice as many as a lone CTA
 // would own, so the 8-row stages divide them better), each its own half of K in one pass; the
 // second CTA stores its sums into the first one's shared memory as it goes, and after one cluster
-// barrier at the end the first CTA adds the two parts and writes y.
+// barrier at the end the first CTA adds the two parts and writes y.  (Another one at the start, its two halves
+// around the filling of the ring, says that the first CTA is there: its shared memory may not be stored to before.)
 //
 // Data path.  One CTA per SM owns a contiguous range of weight rows.  Four producer warps stream
 // them in stages of 8 rows x one K segment with 1-D bulk copies (cp.async.bulk, completion on the
@@ -173,6 +174,7 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if (KS > 1) cluster_arrive();   // waited for before the first sums are sent
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // this CTA's rows and its stages: (pass, row group, segment), row groups of 8 rows
@@ -267,6 +269,8 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
             issue();
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        __syncwarp();
+        if (KS > 1) cluster_wait();
         bool ok = true;
         // the stage whose release is awaited next: ring slot and phase, segment, row group, pass, partial buffer
         int w_slot = 0, w_seg = 0, w_rg = 0, w_pass = 0, w_pbuf = 0;
@@ -310,6 +314,8 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
     const int seg = warp / wps, wi = warp - seg * wps;
 
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    __syncwarp();
+    if (KS > 1) cluster_wait();
     bool ok = true;
     // this warp's next stage: ring slot, full barrier and phase (it takes every nseg-th stage), partial buffer
     int c_slot = seg % S, c_bar = seg, c_pbuf = 0;
@@ -445,7 +451,9 @@ __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(kThreadsMma, 1) q8_
     if (KS > 1) {
         // Every thread of both CTAs gets here, also after a wait that gave up.  The barrier makes the sums
         // the other CTAs stored into the first CTA's shared memory complete and visible; they may leave.
-        cluster_barrier();
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
         if (crank == 0) {
             const int nrows = r_end - r_begin;
             for (int i = threadIdx.x; i < nrows * p.m; i += blockDim.x) {

@@ -57,3 +57,38 @@ def test_only_the_listed_kernels_copy_before_their_wait(fname):
             continue
         wait = first(body, WAIT)
         assert wait is not None and wait < copy, name
+
+
+REMOTE = ("mapa", "shared::cluster.v2.f32", "dsmem_copy(", "mbar_arrive_cluster(")
+CLUSTER_WAIT = ("cluster_wait()", "cluster_sync()")
+
+
+def without_lambdas(body):
+    """The body with its named lambdas taken out, and the names of those that reach another CTA's shared memory."""
+    remote = set()
+    while True:
+        m = re.search(r"auto (\w+) = \[&\]\([^)]*\) \{", body)
+        if m is None:
+            return body, remote
+        depth, j = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(body[j], 0)
+            j += 1
+        if first(body[m.end():j], REMOTE) is not None:
+            remote.add(m.group(1) + "(")
+        body = body[:m.start()] + body[j:]
+
+
+@pytest.mark.parametrize("fname", sorted(f for f in os.listdir(CSRC) if f.endswith(".cu")))
+def test_another_ctas_shared_memory_is_touched_behind_a_cluster_barrier(fname):
+    """A CTA of a cluster may store to another's shared memory, or arrive on its barriers, only once that CTA is known to run: the first
+    half of a cluster barrier before it, and a second barrier that keeps the memory alive until everything has arrived."""
+    for name, body in kernels(fname).items():
+        main, remote = without_lambdas(body)
+        use = first(main, REMOTE + tuple(sorted(remote)))
+        if use is None:
+            continue
+        wait = first(main, CLUSTER_WAIT)
+        assert wait is not None and wait < use, name
+        last_use = max(main.rindex(w) for w in REMOTE + tuple(sorted(remote)) if w in main)
+        assert max(main.rindex(w) for w in CLUSTER_WAIT if w in main) > last_use, name
