@@ -1,0 +1,113 @@
+// How many warps a CTA of the dp4a decode kernels gets, how deep its rings are, and whether weight rows go out in pairs: chosen on the host once per
+// call, in front of launches of a few microseconds.  So a choice costs some 50 ns whatever the shape (tests/test_gemv_plan.py): one division for the ring
+// depths of all counts, and the weights of a count from a table.
+#pragma once
+
+#include <cmath>
+#include <cstddef>
+#include <cstdint>
+
+namespace tpb_gemv {
+
+struct GemvPlan {
+    int warps = 0, stages = 0;   // 0: the activations leave no room
+    bool pairs = false;          // weight rows are dealt out in pairs (warp_row_pairs)
+};
+
+constexpr int kPlanWarps = 20;   // of any kernel
+struct PlanWeights {
+    double inv[kPlanWarps + 1];      // 1 / w
+    double turns[kPlanWarps + 1];    // what w warps cost for filling the SM's four schedulers unevenly
+    double worth[kPlanWarps + 1];    // its inverse, and that more warps hide a little more latency
+    PlanWeights() : inv{}, turns{}, worth{} {
+        for (int w = 1; w <= kPlanWarps; w++) {
+            inv[w] = 1.0 / w;
+            turns[w] = (double)(4 * ((w + 3) / 4)) / w;
+            worth[w] = pow((double)w / kPlanWarps, 0.1) / turns[w];
+        }
+    }
+};
+static const PlanWeights kPlanWeights;
+
+inline double ceil_about(double v) { return (double)(long long)(v + 0.999999); }
+
+// Ring stages (of `stage` bytes and an mbarrier each) that fit beside `act` bytes, over all warps.
+inline int64_t plan_slots(size_t limit, size_t act, size_t stage) {
+    return act + 64 <= limit ? (int64_t)((limit - act - 64) / (stage + 8)) : 0;
+}
+
+// Warps and stages of the Q8_0 dp4a kernels for one rows-per-stage choice (stage = its bytes).  The slowest warp carries
+// ceil(rows / warps_total) rows.  Among the counts that fit (with >= 2 stages and the activations in shared memory) take the one with the best
+// balance; ties go to more warps.  E.g. 5120 rows on 148 SMs: 16 warps -> 2.16 rows per warp (3 vs 2, 72 %), 12 warps -> 2.88 (96 %).
+// Kernels that may have more than sixteen warps deal rows out in pairs, one a step (warp_row_pairs).  What counts then is the share of the
+// warps' steps that is work -- a third of it, as the last steps of the slowest warps run on an SM that is half empty and so faster -- how evenly the warps
+// fill the SM's four schedulers, and a little how many there are.  us at M = 1, at most sixteen warps with ranges cut at any row / so: 5120 x 5120
+// 7.9 / 6.6 (twelve warps with two steps / eighteen with one), 17408 x 5120 17.8 / 17.2, 14336 x 4096 12.3 / 11.9, 5120 x 17408 20.3 / 17.8, 20000 x 2304 18.8 / 13.1,
+// 32000 x 4096 23.3 / 23.3 (on 20 warps 24.3); the f32 kernel 5120 x 5120 10.7 / 9.4, 14336 x 4096 16.5 / 14.8, 17408 x 5120 23.6 / 21.3, 5120 x 17408 27.2 / 21.7.
+// Over 31 shapes of each 1.04 x on average, the worst 0.97.
+inline GemvPlan dp4a_plan(int sms, size_t limit, size_t act, int64_t rows, int stage, int max_warps, int max_stages) {
+    GemvPlan best;
+    const int slots = (int)plan_slots(limit, act, (size_t)stage);
+    const bool pairs = max_warps > 16;
+    const double per_sm = (double)rows / sms;
+    double best_eff = -1.0;
+    for (int w = max_warps; w >= (max_warps < 16 ? max_warps / 2 : 8); w--) {
+        if (2 * w > slots) continue;
+        const double per_warp = per_sm * kPlanWeights.inv[w];
+        double eff = per_warp, margin = 0.02;
+        if (pairs && rows > 2ll * sms * w) {
+            const double n = per_warp * 0.5;
+            eff = n / (0.65 * n + 0.35 * ceil_about(n)) * kPlanWeights.worth[w];
+            margin = 0.0;
+        } else if (rows >= (int64_t)sms * w) {
+            eff = per_warp / ceil_about(per_warp);
+        }
+        if (eff > best_eff + margin) {
+            best_eff = eff;
+            best.warps = w;
+        }
+    }
+    if (best.warps != 0) best.stages = max_stages * best.warps <= slots ? max_stages : slots / best.warps;
+    return best;
+}
+
+// Warps and stages of the dp4a kernels of the other formats.  Every warp owns a contiguous range of whole rows; among the counts that fit with
+// >= 2 stages take the one whose ranges divide most evenly (ties: more warps).
+// With more than one step a warp, rows may be dealt out in pairs (may_pair): the cost of a count is then its average number of steps and, as the last
+// ones run on an SM that is half empty, a third of what the slowest warp has above it, over how evenly the warps fill the four schedulers.  Ranges cut
+// at any row cost half a step a row; pairs are taken where they come out 2 % lower.  us at M = 1, cut / in pairs: 14336 x 4096 q4_k 9.8 (14 warps of 6.92 rows) /
+// 9.1 (16 of 3.03 pairs), q5_k 11.8 / 10.8, q6_k 13.8 / 12.9, iq4_nl 16.5 / 15.4; 5120 x 5120 q4_k 7.2 / 6.8, q6_k 11.7 / 10.7; 13500 x 6144 q4_k 19.9 / 10.8;
+// but 7000 x 3072 (2.96 rows, 1.48 pairs) iq4_nl 9.0 / 9.9, 3072 x 3072 q5_k 4.8 / 5.0.
+inline GemvPlan kq_plan(int sms, size_t limit, size_t act, size_t stage, int64_t rows, int max_stages, bool may_pair) {
+    GemvPlan best;
+    const int slots = (int)plan_slots(limit, act, stage);
+    may_pair = may_pair && rows > 2ll * 16 * sms;
+    const double per_sm = (double)rows / sms;
+    double best_eff = -1.0, cut_cost = 0.0, pair_cost = 0.0;
+    int pair_warps = 0;
+    for (int w = 16; w >= 4; w--) {
+        if (2 * w > slots) continue;
+        const double per_warp = per_sm * kPlanWeights.inv[w], most = ceil_about(per_warp);
+        const double eff = rows >= (int64_t)sms * w ? per_warp / most : per_warp;
+        if (eff > best_eff + 0.02) {
+            best_eff = eff;
+            best.warps = w;
+            cut_cost = 0.5 * most;
+        }
+        if (!may_pair) continue;
+        const double steps = 0.5 * per_warp;
+        const double cost = (0.65 * steps + 0.35 * ceil_about(steps)) * kPlanWeights.turns[w];
+        if (pair_warps == 0 || cost < pair_cost) {
+            pair_cost = cost;
+            pair_warps = w;
+        }
+    }
+    if (may_pair && pair_warps != 0 && pair_cost < 0.98 * cut_cost) {
+        best.warps = pair_warps;
+        best.pairs = true;
+    }
+    if (best.warps != 0) best.stages = max_stages * best.warps <= slots ? max_stages : slots / best.warps;
+    return best;
+}
+
+}  // namespace tpb_gemv

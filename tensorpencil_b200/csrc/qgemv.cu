@@ -19,9 +19,7 @@
 // warp, and y = acc * scale.
 #include <cuda_fp16.h>
 
-#include <cmath>
-
-
+#include "gemv_plan.h"
 #include "qgemv_common.cuh"
 
 using namespace tpb_gemv;
@@ -508,45 +506,6 @@ static GemvOverride gemv_override() {
     return v;
 }
 
-// Warps per CTA and stages per warp of the dp4a kernel for one rows-per-stage choice (stage = its bytes); 0 warps:
-// the activations leave no room.  The slowest warp carries ceil(rows / warps_total) rows.  Among the counts that fit (with >= 2 stages and
-// the activations in shared memory) take the one with the best balance; ties go to more warps.  E.g. 5120 rows on 148 SMs:
-// 16 warps -> 2.16 rows per warp (3 vs 2, 72 %), 12 warps -> 2.88 (96 %).
-// Kernels that may have more than sixteen warps deal rows out in pairs, one a step (warp_row_pairs).  What counts then is the share of the
-// warps' steps that is work -- a third of it, as the last steps of the slowest warps run on an SM that is half empty and so faster -- how evenly the warps
-// fill the SM's four schedulers, and a little how many there are.  us at M = 1, at most sixteen warps with ranges cut at any row / so: 5120 x 5120
-// 7.9 / 6.6 (twelve warps with two steps / eighteen with one), 17408 x 5120 17.8 / 17.2, 14336 x 4096 12.3 / 11.9, 5120 x 17408 20.3 / 17.8, 20000 x 2304 18.8 / 13.1,
-// 32000 x 4096 23.3 / 23.3 (on 20 warps 24.3); the f32 kernel 5120 x 5120 10.7 / 9.4, 14336 x 4096 16.5 / 14.8, 17408 x 5120 23.6 / 21.3, 5120 x 17408 27.2 / 21.7.
-// Over 31 shapes of each 1.04 x on average, the worst 0.97.
-static void dp4a_plan(tpb_handle_t h, size_t act, int64_t rows, int stage, int max_warps, int max_stages, int *warps, int *stages) {
-    const size_t limit = (size_t)h->smem_optin - 1024;
-    *warps = 0;
-    *stages = 0;
-    double best_eff = -1.0;
-    for (int w = max_warps; w >= (max_warps < 16 ? max_warps / 2 : 8); w--) {
-        int s_fit = 0;
-        for (int s = max_stages; s >= 2; s--)
-            if (act + (size_t)w * s * stage + (size_t)w * s * 8 + 64 <= limit) {
-                s_fit = s;
-                break;
-            }
-        if (s_fit == 0) continue;
-        const double per_warp = (double)rows / ((double)h->sm_count * w);
-        double eff = per_warp >= 1.0 ? per_warp / (double)(long long)(per_warp + 0.999999) : per_warp;
-        double margin = 0.02;
-        if (max_warps > 16 && per_warp > 2.0) {
-            const double n = per_warp * 0.5, idle = (double)(long long)(n + 0.999999) - n;
-            eff = n / (n + 0.35 * idle) * ((double)w / (double)(4 * ((w + 3) / 4))) * pow((double)w / max_warps, 0.1);
-            margin = 0.0;
-        }
-        if (eff > best_eff + margin) {
-            best_eff = eff;
-            *warps = w;
-            *stages = s_fit;
-        }
-    }
-}
-
 // Ring depth of the dp4a kernel: two stages where the one that is on its way while a warp works on the other covers the memory's latency,
 // four where it does not.  Sixteen warps with a stage of two whole chunks (4.3 KB) on its way are 70 KB per SM, 10 MB in all, and HBM
 // needs some 6.5 MB (1 us at 6.55 TB/s); what a deeper ring adds is copies that a warp's first lane issues between two steps of
@@ -560,13 +519,18 @@ static int q8n_stages(tpb_handle_t h, int64_t rows, int64_t cols) {
     return cols >= 4096 && rows >= 24 * h->sm_count && bytes < 56e6 ? 2 : 4;
 }
 
+// The plan of the dp4a kernel with two rows per stage, for m activation rows.
+static GemvPlan q8n_plan(tpb_handle_t h, int64_t rows, int64_t cols, int m) {
+    const size_t act = (size_t)m * (size_t)(cols / 64) * kActPairBytes + (size_t)m * (size_t)(cols / 32) * 4;
+    return dp4a_plan(h->sm_count, (size_t)h->smem_optin - 1024, act, rows, stage_bytes(2), q8n_max_warps(m, 2), q8n_stages(h, rows, cols));
+}
+
+// plan2: q8n_plan's answer where the choice of the kernel has asked for it already.
 template <int M, int R>
-int launch_q8n_cfg(tpb_handle_t h, cudaStream_t st, const GemvParams &p, int max_warps) {
+int launch_q8n_cfg(tpb_handle_t h, cudaStream_t st, const GemvParams &p, int max_warps, const GemvPlan *plan2) {
     constexpr int kStage = stage_bytes(R);
     const size_t limit = (size_t)h->smem_optin - 1024;
     const size_t act = (size_t)M * (p.nblk / 2) * kActPairBytes + (size_t)M * p.nblk * 4;
-    int warps = 0, stages = 0;
-    bool act_smem = true;
     const GemvOverride ov = gemv_override();
     if (ov.r == R && ov.warps > 0 && ov.warps <= max_warps && ov.stages >= 2) {
         const size_t need = act + (size_t)ov.warps * ov.stages * kStage + (size_t)ov.warps * ov.stages * 8 + 64;
@@ -579,7 +543,10 @@ int launch_q8n_cfg(tpb_handle_t h, cudaStream_t st, const GemvParams &p, int max
         TPB_CUDA(h, launch_pdl(kern, grid, ov.warps * 32, need, st, p, ov.stages));
         return TPB_OK;
     }
-    dp4a_plan(h, act, p.rows, kStage, max_warps, q8n_stages(h, p.rows, p.cols), &warps, &stages);
+    const GemvPlan pl = R == 2 ? (plan2 != nullptr ? *plan2 : q8n_plan(h, p.rows, p.cols, M))
+                               : dp4a_plan(h->sm_count, limit, act, p.rows, kStage, max_warps, q8n_stages(h, p.rows, p.cols));
+    int warps = pl.warps, stages = pl.stages;
+    bool act_smem = true;
     if (stages == 0) {
         if (R == 2) return TPB_ERR_STATE;
         act_smem = false;
@@ -608,7 +575,7 @@ int launch_q8n_cfg(tpb_handle_t h, cudaStream_t st, const GemvParams &p, int max
 }
 
 template <int M>
-int launch_q8n(tpb_handle_t h, cudaStream_t st, const GemvParams &p) {
+int launch_q8n(tpb_handle_t h, cudaStream_t st, const GemvParams &p, const GemvPlan *plan2) {
     const size_t row_bytes = (size_t)p.nblk * kBlockBytes;
     if (row_bytes % 16 != 0) {
         const int block = 256;
@@ -617,14 +584,14 @@ int launch_q8n(tpb_handle_t h, cudaStream_t st, const GemvParams &p) {
         TPB_CUDA(h, cudaGetLastError());
         return TPB_OK;
     }
-    // Preferred: up to 16 warps with 2 weight rows each (more loads in flight, more latency
+    // Preferred: up to 16 warps (20 for one and two activation rows) with 2 weight rows each (more loads in flight, more latency
     // hiding).  When the activations leave too little shared memory for that, 8 warps with
     // 4 rows each (activations are re-read from shared memory once per R rows).
     if (gemv_override().r != 4) {
-        const int rc = launch_q8n_cfg<M, 2>(h, st, p, q8n_max_warps(M, 2));
+        const int rc = launch_q8n_cfg<M, 2>(h, st, p, q8n_max_warps(M, 2), plan2);
         if (rc != TPB_ERR_STATE) return rc;  // TPB_ERR_STATE: did not fit, try the wider grouping
     }
-    return launch_q8n_cfg<M, 4>(h, st, p, 8);
+    return launch_q8n_cfg<M, 4>(h, st, p, 8, nullptr);
 }
 
 }  // namespace
@@ -657,6 +624,8 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
     // them a warp for two-row stages; eighteen warps with one step each take 17.8 and 18.8 for one and two activation rows);  32000 x 4096  22.6 22.7 24.8 26.7 29.9 / 27.1-28.7;  4096 x 14336  11.6 12.7 13.7 15.1
     // 16.9 26.7 / 15.3-16.2;  8192 x 28672  41.0 42.2 69.6 / 49.8-53.0;  28672 x 8192  41.4 42.4 43.6 47.9 /
     // 41.4-44.9.  The rule below follows that table.  TPB_GEMV_KERNEL=dp4a / mma forces one.
+    GemvPlan plan;
+    bool planned = false;
     {
         const char *e = getenv("TPB_GEMV_KERNEL");
         const bool force_dp4a = e != nullptr && e[0] == 'd', force_mma = e != nullptr && e[0] == 'm';
@@ -667,8 +636,9 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
         if (mma_ks != 0 && !force_mma) {
             // the dp4a kernel at its best: fourteen warps with two two-row stages each fit beside the activations
             // (with fewer its time jumps: K = 14336 from the sixth activation row on, K = 28672 from the third)
-            int warps = 0, stages = 0;
-            dp4a_plan(h, act_bytes, rows, stage_bytes(2), q8n_max_warps(ng, 2), q8n_stages(h, rows, cols), &warps, &stages);
+            plan = q8n_plan(h, rows, cols, ng);
+            planned = true;
+            const int warps = plan.warps;
             const bool roomy = warps != 0 && act_bytes + 14 * 2 * (size_t)stage_bytes(2) + 14 * 2 * 8 + 64 <=
                                                  (size_t)h->smem_optin - 1024;
             // share of its row slots that hold a row: rows come to a warp two at a time
@@ -704,14 +674,14 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
     p.nblk = nblk;
     p.status = h->d_status;
     switch (ng) {
-        case 1: return launch_q8n<1>(h, st, p);
-        case 2: return launch_q8n<2>(h, st, p);
-        case 3: return launch_q8n<3>(h, st, p);
-        case 4: return launch_q8n<4>(h, st, p);
-        case 5: return launch_q8n<5>(h, st, p);
-        case 6: return launch_q8n<6>(h, st, p);
-        case 7: return launch_q8n<7>(h, st, p);
-        case 8: return launch_q8n<8>(h, st, p);
+        case 1: return launch_q8n<1>(h, st, p, planned ? &plan : nullptr);
+        case 2: return launch_q8n<2>(h, st, p, planned ? &plan : nullptr);
+        case 3: return launch_q8n<3>(h, st, p, planned ? &plan : nullptr);
+        case 4: return launch_q8n<4>(h, st, p, planned ? &plan : nullptr);
+        case 5: return launch_q8n<5>(h, st, p, planned ? &plan : nullptr);
+        case 6: return launch_q8n<6>(h, st, p, planned ? &plan : nullptr);
+        case 7: return launch_q8n<7>(h, st, p, planned ? &plan : nullptr);
+        case 8: return launch_q8n<8>(h, st, p, planned ? &plan : nullptr);
     }
     return tpb_fail(h, TPB_ERR_INVALID_ARG, "q8_0_gemv_q8n: ng out of range");
 }
@@ -729,8 +699,8 @@ int tpb_launch_q8_0_gemv_f32(tpb_handle_t h, cudaStream_t st, float *y, const fl
     // shapes within 1 %.
     if (cols % 256 == 0 && cols >= (rows < 64 ? 2048 : 1024)) {
         const size_t act = (size_t)(cols / 64) * kF32PairBytes;
-        int warps = 0, stages = 0;
-        dp4a_plan(h, act, rows, stage_bytes(2), kF32Warps, 2, &warps, &stages);
+        const GemvPlan pl = dp4a_plan(h->sm_count, (size_t)h->smem_optin - 1024, act, rows, stage_bytes(2), kF32Warps, 2);
+        const int warps = pl.warps, stages = pl.stages;
         if (warps != 0) {
             int rgrid = (int)((rows + 2 * warps - 1) / (2 * warps));
             if (rgrid > h->sm_count) rgrid = h->sm_count;

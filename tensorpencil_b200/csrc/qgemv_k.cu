@@ -27,6 +27,7 @@
 // which is what the kernels accumulate in f32.
 #include <cuda_fp16.h>
 
+#include "gemv_plan.h"
 #include "qgemv_common.cuh"
 
 using namespace tpb_gemv;
@@ -867,48 +868,8 @@ static size_t kq_stage_bytes(int fmt, int ng, int64_t cols) {
     if (fmt == TPB_GGUF_Q6_K) return 2 * (size_t)kQ6RowStage;
     return 2 * (size_t)32 * (kq_three_units(ng, cols) ? 3 : 2) * (fmt == TPB_GGUF_Q5_K ? 44 : 36);
 }
-// Warps per CTA: every warp owns a contiguous range of whole rows; among the counts that fit with >= 2 stages take the one whose
-// ranges divide most evenly (ties: more warps).
-// With more than one step a warp, rows may be dealt out in pairs (pairs != null): the cost of a count is then its average number of steps and, as the last
-// ones run on an SM that is half empty, a third of what the slowest warp has above it, over how evenly the warps fill the four schedulers.  Ranges cut
-// at any row cost half a step a row; pairs are taken where they come out 2 % lower.  us at M = 1, cut / in pairs: 14336 x 4096 q4_k 9.8 (14 warps of 6.92 rows) /
-// 9.1 (16 of 3.03 pairs), q5_k 11.8 / 10.8, q6_k 13.8 / 12.9, iq4_nl 16.5 / 15.4; 5120 x 5120 q4_k 7.2 / 6.8, q6_k 11.7 / 10.7; 13500 x 6144 q4_k 19.9 / 10.8;
-// but 7000 x 3072 (2.96 rows, 1.48 pairs) iq4_nl 9.0 / 9.9, 3072 x 3072 q5_k 4.8 / 5.0.
-static void kq_plan(tpb_handle_t h, size_t act, size_t stage, int64_t rows, int max_stages, int *warps, int *stages, bool *pairs) {
-    const size_t limit = (size_t)h->smem_optin - 1024;
-    *warps = *stages = 0;
-    double best_eff = -1.0, cut_cost = 0.0, pair_cost = 0.0;
-    int pair_warps = 0, pair_stages = 0;
-    for (int w = 16; w >= 4; w--) {
-        int s_fit = 0;
-        for (int s = max_stages; s >= 2; s--)
-            if (act + (size_t)w * s * stage + (size_t)w * s * 8 + 64 <= limit) {
-                s_fit = s;
-                break;
-            }
-        if (s_fit == 0) continue;
-        const double per_warp = (double)rows / ((double)h->sm_count * w), most = (double)(long long)(per_warp + 0.999999);
-        const double eff = per_warp >= 1.0 ? per_warp / most : per_warp;
-        if (eff > best_eff + 0.02) {
-            best_eff = eff;
-            *warps = w;
-            *stages = s_fit;
-            cut_cost = 0.5 * most;
-        }
-        const double steps = 0.5 * per_warp, top = (double)(long long)(steps + 0.999999);
-        const double cost = (steps + 0.35 * (top - steps)) * (double)(4 * ((w + 3) / 4)) / w;
-        if (pair_warps == 0 || cost < pair_cost) {
-            pair_cost = cost;
-            pair_warps = w;
-            pair_stages = s_fit;
-        }
-    }
-    if (pairs == nullptr) return;
-    *pairs = rows > 2ll * 16 * h->sm_count && pair_warps != 0 && pair_cost < 0.98 * cut_cost;
-    if (*pairs) {
-        *warps = pair_warps;
-        *stages = pair_stages;
-    }
+static GemvPlan kq_warps(tpb_handle_t h, size_t act, size_t stage, int64_t rows, int max_stages, bool may_pair) {
+    return kq_plan(h->sm_count, (size_t)h->smem_optin - 1024, act, stage, rows, max_stages, may_pair);
 }
 
 // Ring depth of the dp4a kernel of q4_0, iq4_nl, q4_k and q5_k: two stages from 14 MB on.  A warp's copies are issued by its first lane
@@ -934,9 +895,8 @@ static int kq_max_stages(int64_t rows, size_t row_bytes) { return (double)rows *
 static bool mma_wins(tpb_handle_t h, int fmt, int64_t rows, int64_t cols, int m) {
     const int64_t weights = rows * cols;
     if (m < 3 || weights < 5000000) return false;
-    int warps = 0, stages = 0;
     const int max_stages = fmt == TPB_GGUF_Q6_K ? 4 : kq_max_stages(rows, tpb_gguf_row_bytes(fmt, cols));
-    kq_plan(h, kq_act_bytes(fmt, m, cols), kq_stage_bytes(fmt, m, cols), rows, max_stages, &warps, &stages, nullptr);
+    const int warps = kq_warps(h, kq_act_bytes(fmt, m, cols), kq_stage_bytes(fmt, m, cols), rows, max_stages, false).warps;
     if (warps <= 5 && weights >= 20000000) return true;
     const double per_cta = (double)rows / h->sm_count > 4.0 ? (double)rows / h->sm_count : 4.0;
     const double fill = per_cta / (16.0 * (double)((long long)(per_cta / 16.0 + 0.999999)));
@@ -984,9 +944,8 @@ int launch_q6k_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     }
     constexpr int kStage = R * kQ6RowStage;
     const size_t act = kq_act_bytes(TPB_GGUF_Q6_K, M, p.cols);
-    int warps = 0, stages = 0;
-    bool pairs = false;
-    kq_plan(h, act, kStage, p.rows, 4, &warps, &stages, kq_pairs(M) ? &pairs : nullptr);
+    const GemvPlan pl = kq_warps(h, act, kStage, p.rows, 4, kq_pairs(M));
+    const int warps = pl.warps, stages = pl.stages;
     if (stages == 0)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "gguf_gemv: %d activation rows of %d columns do not fit shared memory",
                         M, p.cols);
@@ -998,7 +957,7 @@ int launch_q6k_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     static tpb_per_device_once smem_set;   // the size varies per call: opt in to the device maximum, once
     TPB_CUDA(h, tpb_set_max_smem_once(h, kern, h->smem_optin, smem_set));
     KGemvParams pp = p;
-    pp.pairs = pairs;
+    pp.pairs = pl.pairs;
     TPB_CUDA(h, tpb_launch_pdl(kern, dim3(grid), dim3(warps * 32), smem, st, pp, stages));
     return TPB_OK;
 }
@@ -1022,9 +981,8 @@ int launch_fmt_mu(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     constexpr int R = 2;
     constexpr int kStage = R * 32 * U * Fmt<FMT>::kUnitBytes;
     const size_t act = (size_t)M * (p.cols / 64) * kActPairBytes + (size_t)M * p.nblk * 8;
-    int warps = 0, stages = 0;
-    bool pairs = false;
-    kq_plan(h, act, kStage, p.rows, kq_max_stages(p.rows, p.row_bytes), &warps, &stages, kq_pairs(M) ? &pairs : nullptr);
+    const GemvPlan pl = kq_warps(h, act, kStage, p.rows, kq_max_stages(p.rows, p.row_bytes), kq_pairs(M));
+    const int warps = pl.warps, stages = pl.stages;
     if (stages == 0)
         return tpb_fail(h, TPB_ERR_INVALID_ARG, "gguf_gemv: %d activation rows of %d columns do not fit shared memory",
                         M, p.cols);
@@ -1036,7 +994,7 @@ int launch_fmt_mu(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     static tpb_per_device_once smem_set;   // the size varies per call: opt in to the device maximum, once
     TPB_CUDA(h, tpb_set_max_smem_once(h, kern, h->smem_optin, smem_set));
     KGemvParams pp = p;
-    pp.pairs = pairs;
+    pp.pairs = pl.pairs;
     TPB_CUDA(h, tpb_launch_pdl(kern, dim3(grid), dim3(warps * 32), smem, st, pp, stages));
     return TPB_OK;
 }
