@@ -44,7 +44,9 @@ inline int64_t plan_slots(size_t limit, size_t act, size_t stage) {
 // fill the SM's four schedulers, and a little how many there are.  us at M = 1, at most sixteen warps with ranges cut at any row / so: 5120 x 5120
 // 7.9 / 6.6 (twelve warps with two steps / eighteen with one), 17408 x 5120 17.8 / 17.2, 14336 x 4096 12.3 / 11.9, 5120 x 17408 20.3 / 17.8, 20000 x 2304 18.8 / 13.1,
 // 32000 x 4096 23.3 / 23.3 (on 20 warps 24.3); the f32 kernel 5120 x 5120 10.7 / 9.4, 14336 x 4096 16.5 / 14.8, 17408 x 5120 23.6 / 21.3, 5120 x 17408 27.2 / 21.7.
-// Over 31 shapes of each 1.04 x on average, the worst 0.97.
+// More than sixteen only where each of them gets more than one row: a CTA is launched for every two rows a warp, so a count that leaves warps with one row
+// leaves SMs without a CTA (2500 rows on eighteen warps a CTA: 70 CTAs, on nine 139; us, eighteen / nine: f32 2504 x 8704 11.5 / 9.1, 2746 x 11264 13.4 /
+// 10.4, Q8_0 at M = 2 2372 x 9216 9.2 / 7.7).
 inline GemvPlan dp4a_plan(int sms, size_t limit, size_t act, int64_t rows, int stage, int max_warps, int max_stages) {
     GemvPlan best;
     const int slots = (int)plan_slots(limit, act, (size_t)stage);
@@ -52,7 +54,7 @@ inline GemvPlan dp4a_plan(int sms, size_t limit, size_t act, int64_t rows, int s
     const double per_sm = (double)rows / sms;
     double best_eff = -1.0;
     for (int w = max_warps; w >= (max_warps < 16 ? max_warps / 2 : 8); w--) {
-        if (2 * w > slots) continue;
+        if (2 * w > slots || (w > 16 && rows <= (int64_t)sms * w)) continue;
         const double per_warp = per_sm * kPlanWeights.inv[w];
         double eff = per_warp, margin = 0.02;
         if (pairs && rows > 2ll * sms * w) {

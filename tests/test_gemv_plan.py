@@ -68,7 +68,7 @@ def q8(act, rows, max_warps, max_stages):
     best, pick = -1.0, (0, 0)
     for w in range(max_warps, 7, -1):
         s = fits(act, w, 4352, max_stages)
-        if not s:
+        if not s or (w > 16 and rows <= SMS * w):
             continue
         per = rows / (SMS * w)
         eff, margin = (per / int(per + 0.999999) if per >= 1 else per), 0.02
@@ -108,6 +108,17 @@ def test_choice_is_the_formulas(plan, act):
             got = tuple(int(v) for v in next(lines).split())
             want = q8(act, rows, 20, stages) + q8(act, rows, 16, stages) + kq(act, rows, stages, True) + kq(act, rows, stages, False)[:2]
             assert got == want, (rows, stages)
+
+
+@pytest.mark.parametrize("act", [2880, 48960])
+def test_more_warps_do_not_leave_sms_without_a_cta(plan, act):
+    """A CTA is launched for every two rows a warp: with up to twenty warps at least as many of them as with up to sixteen, but for a tenth."""
+    ctas = lambda rows, warps: min(SMS, -(-rows // (2 * warps)))
+    lines = iter(plan(1, 9000, 3, act).split("\n"))
+    for rows in range(1, 9000, 3):
+        for _ in range(2):
+            got = [int(v) for v in next(lines).split()]
+            assert ctas(rows, got[0]) >= 0.9 * ctas(rows, got[2]), rows
 
 
 def test_choice_costs_about_the_same_for_every_shape(plan):
