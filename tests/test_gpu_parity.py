@@ -294,6 +294,18 @@ def test_w4_expand_matches_nibble_decode(be):
     assert np.array_equal(out.cpu().numpy(), w)
 
 
+@pytest.mark.parametrize("n,k", [(1, 32), (3, 544), (33, 1024), (63, 1056), (11839, 1024), (11840, 1024), (11841, 1056)])
+def test_w4_expand_at_the_edges_of_its_ctas(be, n, k):
+    """One piece, whole CTAs and remainders of two and of four pieces a thread (on 148 SMs the line is 11840 x 1024), and nothing behind the weight."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    out = torch.full((n * k + 64,), 77, dtype=torch.int8, device="cuda")
+    assert be.lib.tpb_convrot_w4_expand(be.h, be._stream(), packed.data_ptr(), n, k, out.data_ptr()) == 0
+    nib = torch.stack([packed & 15, packed >> 4], dim=-1).flatten().to(torch.int8)
+    assert torch.equal(out[: n * k], nib - 16 * (nib > 7).to(torch.int8))
+    assert bool((out[n * k:] == 77).all())
+
+
 # ---------------------------------------------------------------------------------
 # K4: Q8_0 GEMV
 # ---------------------------------------------------------------------------------
