@@ -75,18 +75,21 @@ inline GemvPlan dp4a_plan(int sms, size_t limit, size_t act, int64_t rows, int s
 
 // Warps and stages of the dp4a kernels of the other formats.  Every warp owns a contiguous range of whole rows; among the counts that fit with
 // >= 2 stages take the one whose ranges divide most evenly (ties: more warps).
-// With more than one step a warp, rows may be dealt out in pairs (may_pair): the cost of a count is then its average number of steps and, as the last
-// ones run on an SM that is half empty, a third of what the slowest warp has above it, over how evenly the warps fill the four schedulers.  Ranges cut
-// at any row cost half a step a row; pairs are taken where they come out 2 % lower.  us at M = 1, cut / in pairs: 14336 x 4096 q4_k 9.8 (14 warps of 6.92 rows) /
-// 9.1 (16 of 3.03 pairs), q5_k 11.8 / 10.8, q6_k 13.8 / 12.9, iq4_nl 16.5 / 15.4; 5120 x 5120 q4_k 7.2 / 6.8, q6_k 11.7 / 10.7; 13500 x 6144 q4_k 19.9 / 10.8;
-// but 7000 x 3072 (2.96 rows, 1.48 pairs) iq4_nl 9.0 / 9.9, 3072 x 3072 q5_k 4.8 / 5.0.
+// With one or two activation rows and more than one step a warp, rows may be dealt out in pairs, one a step (may_pair): to the number of warps whose cost is
+// lowest, its average number of steps and, as the last ones run on an SM that is half empty, a third of what the slowest warp has above it, over how
+// evenly the warps fill the four schedulers.  What decides between ranges and pairs is the steps of the slowest warp: pairs are taken
+// where they have fewer of them, and with the same number from five on, or from three where the ranges come out at thirteen or fourteen
+// warps, which leave schedulers with three warps beside some with four.  Ranges / pairs over 300 shapes and formats at M = 1 and 2, by the slowest warp's steps: 9 / 3
+// 1.5 x, 5 / 4 1.07, 3 / 2 1.08, 5 / 5 1.03, 4 / 4 and 3 / 3 on 13 and 14 warps 1.03, 3 / 3 on others 0.94, 2 / 2 0.96; over 300 others the rule's worst choice
+// has 0.96.  us at M = 1: 14336 x 4096 q4_k 9.8 (14 warps of 6.92 rows) / 9.1 (16 of 3.03 pairs), q5_k 11.8 / 10.8, q6_k 13.8 / 12.9, iq4_nl 16.5 / 15.4; 13500 x
+// 6144 q4_k 19.9 / 10.8; but 10638 x 5632 q6_k (12 of 5.99, 16 of 2.25 pairs) 14.8 / 17.3, 5907 x 1280 q5_k (10 of 3.99, 16 of 1.25) 4.5 / 5.4.
 inline GemvPlan kq_plan(int sms, size_t limit, size_t act, size_t stage, int64_t rows, int max_stages, bool may_pair) {
     GemvPlan best;
     const int slots = (int)plan_slots(limit, act, stage);
     may_pair = may_pair && rows > 2ll * 16 * sms;
     const double per_sm = (double)rows / sms;
-    double best_eff = -1.0, cut_cost = 0.0, pair_cost = 0.0;
-    int pair_warps = 0;
+    double best_eff = -1.0, pair_cost = 0.0;
+    int cut_steps = 0, pair_warps = 0, pair_steps = 0;      // steps: of the slowest warp
     for (int w = 16; w >= 4; w--) {
         if (2 * w > slots) continue;
         const double per_warp = per_sm * kPlanWeights.inv[w], most = ceil_about(per_warp);
@@ -94,17 +97,19 @@ inline GemvPlan kq_plan(int sms, size_t limit, size_t act, size_t stage, int64_t
         if (eff > best_eff + 0.02) {
             best_eff = eff;
             best.warps = w;
-            cut_cost = 0.5 * most;
+            cut_steps = ((int)most + 1) / 2;
         }
         if (!may_pair) continue;
-        const double steps = 0.5 * per_warp;
-        const double cost = (0.65 * steps + 0.35 * ceil_about(steps)) * kPlanWeights.turns[w];
+        const double steps = 0.5 * per_warp, top = ceil_about(steps);
+        const double cost = (0.65 * steps + 0.35 * top) * kPlanWeights.turns[w];
         if (pair_warps == 0 || cost < pair_cost) {
             pair_cost = cost;
             pair_warps = w;
+            pair_steps = (int)top;
         }
     }
-    if (may_pair && pair_warps != 0 && pair_cost < 0.98 * cut_cost) {
+    const int same_from = best.warps == 13 || best.warps == 14 ? 3 : 5;
+    if (pair_warps != 0 && (pair_steps < cut_steps || (pair_steps == cut_steps && pair_steps >= same_from))) {
         best.warps = pair_warps;
         best.pairs = true;
     }
