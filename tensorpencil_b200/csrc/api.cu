@@ -57,6 +57,15 @@ int tpb_create(tpb_handle_t *out, int device_ordinal) {
     const char *e1 = getenv("TPB_W4_FUSED"), *e2 = getenv("TPB_GEMM_ONE_CTA");
     h->opt_w4_fused = e1 != nullptr && e1[0] == '1';
     h->opt_gemm_one_cta = e2 != nullptr && e2[0] == '1';
+    if (const char *e4 = getenv("TPB_GEMM_SPLIT")) {
+        int bn = 0, parts = 0;
+        if (sscanf(e4, "%d,%d", &bn, &parts) == 2 && (bn == 64 || bn == 128 || bn == 192) && parts >= 2 && parts <= 8) {
+            h->opt_gemm_split_bn = bn;
+            h->opt_gemm_split_parts = parts;
+        } else if (e4[0] == '0') {
+            h->opt_gemm_split_bn = 0;
+        }
+    }
     if (const char *e3 = getenv("TPB_GEMM_ABLATE")) h->opt_gemm_ablate = atoi(e3) & 31;
     int prev = 0;
     cudaGetDevice(&prev);

@@ -300,6 +300,15 @@ Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta
     Split best;
     double t_best = 0.96 * one_cta_us;
     const int64_t blocks = k / BK;
+    if (h->opt_gemm_one_cta || h->opt_gemm_split_bn == 0) return best;
+    if (h->opt_gemm_split_bn > 0) {
+        const int64_t tiles = (m + BM - 1) / BM * ((n + h->opt_gemm_split_bn - 1) / h->opt_gemm_split_bn);
+        if (h->opt_gemm_split_parts <= blocks && tiles <= h->max_clusters[h->opt_gemm_split_parts]) {
+            best.bn = h->opt_gemm_split_bn;
+            best.parts = h->opt_gemm_split_parts;
+        }
+        return best;
+    }
     const double rows = (double)(m < BM ? m : BM) / BM;
     for (const auto &c : kCost) {
         const int64_t tiles = (m + BM - 1) / BM * ((n + c.bn - 1) / c.bn);
@@ -382,14 +391,14 @@ int tpb_launch_gemm(tpb_handle_t h, cudaStream_t st, void *y, int y_dtype, int64
         if (rc != TPB_OK) return rc;
         w8 = buf;
     }
-    // TPB_GEMM_ONE_CTA=1 keeps the one-CTA kernel for comparisons.
+    // TPB_GEMM_ONE_CTA=1 keeps the one-CTA kernel for comparisons, TPB_GEMM_SPLIT=0 or "columns,parts" whether and how K is split.
     Tile tile;
     if (n_peers > 0 || mc_y != nullptr) {
         tile = pick_tile_peers(h, m, n);
     } else {
         double us = 0.0;
         tile = pick_tile(h, gate ? EPI_GATED : y_dtype == TPB_BF16 ? EPI_BF16 : EPI_F32, m, n, k, &us);
-        const Split split = pick_split(h, m, n, k, us);
+        const Split split = pick_split(h, m, n, k, us);   // (one part under TPB_GEMM_ONE_CTA)
         if (split.parts > 1) return tpb_launch_gemm_splitk(h, st, p, y_dtype, q, w8, split.bn, split.parts);
     }
     if (tile == P256) return tpb_launch_gemm2(h, st, p, y_dtype, q, w8, false);

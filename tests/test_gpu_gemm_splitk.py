@@ -48,3 +48,123 @@ def test_split_is_exact(be, m, n, k):
     be.status_poll()
     want = x.double() + gate.double() * f32.double()             # the product is exact in f64
     assert bool(((xd.cpu().double() - want).abs() <= 2.0 ** -24 * want.abs() * (1 + 1e-6) + 1e-45).all())   # one rounding to f32
+
+
+# -- every width and cluster size, and which one a call takes ------------------------------------
+
+
+def _kernels(fn):
+    """(name, CTAs) of every kernel that fn launches, from the nodes of a captured graph."""
+    import ctypes as C
+
+    class Params(C.Structure):
+        _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("shared", C.c_uint), ("params", C.c_void_p),
+                    ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+    cu = C.CDLL("libcuda.so.1")
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g, stream=stream):
+            fn()
+        n = C.c_size_t(0)
+        raw = C.c_void_p(g.raw_cuda_graph())
+        assert cu.cuGraphGetNodes(raw, None, C.byref(n)) == 0
+        nodes = (C.c_void_p * n.value)()
+        assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
+        out = []
+        for node in nodes:
+            p, name = Params(), C.c_char_p()
+            if cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) != 0:
+                continue
+            get, arg = (cu.cuFuncGetName, p.func) if p.func else (cu.cuKernelGetName, p.kern)
+            assert get(C.byref(name), C.c_void_p(arg)) == 0
+            out.append((name.value.decode(), p.grid[0]))
+    torch.cuda.synchronize()
+    return out
+
+
+def _split_of(be, y, wd, wsd, n):
+    """(columns, parts) of the GEMM that be._gemm launches for y; None: K in one chain."""
+    (name, ctas), = _kernels(lambda: be._gemm(y, wd, wsd, n, 8))
+    if "splitk" not in name:
+        return None
+    bn = next(b for b in (64, 128, 192) if f"splitk_kernelILi{b}E" in name)
+    tiles = -(-y.shape[0] // 128) * -(-n // bn)
+    assert ctas % tiles == 0
+    return bn, ctas // tiles
+
+
+def _problem(be, m, n, k):
+    rng = np.random.default_rng(m + n + k)
+    q = rng.integers(-127, 128, size=(m, k), dtype=np.int8)
+    w = rng.integers(-128, 128, size=(n, k), dtype=np.int8)
+    s = rng.uniform(0.5, 1.5, m).astype(np.float32)
+    ws = rng.uniform(0.5, 1.5, n).astype(np.float32)
+    acc = oracle.igemm_s32(q, w)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    be.i8_x, be.i8_scale, be.i8_sum = dev(q.reshape(-1)), dev(s), dev(np.zeros(m, np.int32))
+    be.i8_m, be.i8_cols, be.i8_bits = m, k, 8
+    f32 = torch.from_numpy((acc.astype(np.float32) * s[:, None]) * ws[None, :])
+    return dev(w), dev(ws), {torch.int32: torch.from_numpy(acc), torch.float32: f32, torch.bfloat16: f32.to(torch.bfloat16)}
+
+
+def _check(be, m, n, k, wd, wsd, want):
+    for dt, ref in want.items():
+        y = torch.full((m + 1, n + 8), 3, dtype=dt, device="cuda")
+        be._gemm(y, wd, wsd, n, 8, ldy=n + 8)
+        be.status_poll()
+        assert torch.equal(y[:m, :n].cpu(), ref), dt
+        assert bool((y[m] == 3).all()) and bool((y[:, n:] == 3).all())
+    x = torch.randn((m, n), generator=torch.Generator().manual_seed(m))
+    gate = torch.linspace(-1, 1, n)
+    xd = x.cuda()
+    be.gemmGatedAdd(xd, wd, wsd, n, gate.cuda(), 0, 8)
+    be.status_poll()
+    ref = x.double() + gate.double() * want[torch.float32].double()
+    assert bool(((xd.cpu().double() - ref).abs() <= 2.0 ** -24 * ref.abs() * (1 + 1e-6) + 1e-45).all())   # one rounding to f32
+
+
+def _backend(monkeypatch, **env):
+    from tensorpencil_b200.backend import Backend
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    b = Backend(0)
+    for k in env:
+        monkeypatch.delenv(k)
+    return b
+
+
+@pytest.mark.parametrize("parts", range(2, 9))
+@pytest.mark.parametrize("bn", [64, 128, 192])
+def test_every_width_and_cluster_is_exact(monkeypatch, bn, parts):
+    """K of ten blocks, which most clusters do not divide; columns that end inside a tile of each width; fewer rows than CTAs, a tile with
+    rows missing, and a second tile with few."""
+    b = _backend(monkeypatch, TPB_GEMM_SPLIT=f"{bn},{parts}")
+    for m in (1, 5, 100, 133, 200):
+        n, k = 336, 1280
+        wd, wsd, want = _problem(b, m, n, k)
+        assert _split_of(b, torch.empty((m, n), device="cuda"), wd, wsd, n) == (bn, parts)
+        _check(b, m, n, k, wd, wsd, want)
+    b.close()
+
+
+@pytest.mark.parametrize("m,n,k,bn", [(16, 1024, 12288, None), (64, 3072, 6144, None), (256, 3072, 3072, 128), (5, 9552, 512, 192), (16, 12288, 12288, 192)])
+def test_the_rule_splits_long_chains(be, m, n, k, bn):
+    """(More than two CTAs to a cluster: how many clusters the device holds decides the width, too.)"""
+    wd, wsd, want = _problem(be, m, n, k)
+    split = _split_of(be, torch.empty((m, n), device="cuda"), wd, wsd, n)
+    assert split is not None and bn in (None, split[0])
+    _check(be, m, n, k, wd, wsd, want)
+
+
+@pytest.mark.parametrize("env", [{"TPB_GEMM_SPLIT": "0"}, {"TPB_GEMM_ONE_CTA": "1"}])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 256), (7, 48, 256), (129, 80, 512), (200, 272, 768), (300, 1040, 512), (70, 96, 256), (130, 1040, 512), (100, 5008, 256),
+                                   (256, 3072, 3072)])
+def test_one_chain_is_kept_where_asked_for(monkeypatch, env, m, n, k):
+    """Both switches keep K in one chain, and the one-chain kernels are exact on the small shapes that would be split."""
+    b = _backend(monkeypatch, **env)
+    wd, wsd, want = _problem(b, m, n, k)
+    assert _split_of(b, torch.empty((m, n), device="cuda"), wd, wsd, n) is None
+    _check(b, m, n, k, wd, wsd, want)
+    b.close()
