@@ -232,8 +232,9 @@ __device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
 // UPW = units (pairs of groups) per half-warp (compile time, sizes the register file use).
 // ONE_WARP: the row fits one warp (k <= 1024): every warp of the CTA takes its own row and
 // no CTA-wide barrier or shared reduction is needed; otherwise one row per CTA.
-// AHEAD: the kernel can ask rows into L2 (P.ahead).  Stand-alone RMS norm over few rows, which asks for none, has a variant without: 18 x 11008 bf16
-// 4.5 -> 4.3 us, 77 x 9216 f32 6.1 -> 5.8.
+// AHEAD: the kernel can ask rows into L2 (P.ahead).  RMS norm over few rows, which asks for none, has a variant without: alone 18 x 11008 bf16
+// 4.5 -> 4.3 us, 77 x 9216 f32 6.1 -> 5.8; in front of the quantiser with f32 inputs it takes 64 registers a thread instead of 72, so that an eighth
+// CTA of four warps fits an SM (1170 x 3328 11.3 -> 10.1 us).
 template <typename T, int UPW, int OP, bool ACT_ONLY, bool ONE_WARP, bool AHEAD = true>
 __global__ void __launch_bounds__((UPW == 1 ? kMaxWarpsWide : kMaxWarps) * 32)
 convrot_prep_kernel(const PrepParams P) {
@@ -521,12 +522,13 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
         const int64_t wave = (int64_t)rows_per_sm * h->sm_count;
         P.ahead = (sizeof(T) == 2 || OP == OP_RMS_MOD) && m >= 5 * wave ? (int)(wave / 2) : 0;
     };
+    constexpr bool kRms = OP == OP_RMS_MOD;
     cudaError_t err = cudaSuccess;
     if (n_units <= 2) {
         const dim3 grid((unsigned)((m + kRowsPerCta - 1) / kRowsPerCta)), block(kRowsPerCta * 32);
         set_ahead(32);
         const size_t smem = ACT_ONLY ? 0 : (size_t)kRowsPerCta * 2 * kTilePairs * sizeof(f2);
-        auto kern = ACT_ONLY && P.ahead == 0 ? convrot_prep_kernel<T, 1, OP, ACT_ONLY, true, !ACT_ONLY> : convrot_prep_kernel<T, 1, OP, ACT_ONLY, true>;
+        auto kern = kRms && P.ahead == 0 ? convrot_prep_kernel<T, 1, OP, ACT_ONLY, true, !kRms> : convrot_prep_kernel<T, 1, OP, ACT_ONLY, true>;
         err = tpb_launch_pdl(kern, grid, block, smem, st, P);
     } else {
         // One unit per half-warp, up to 16 warps a row, where the row fits that way (k <= 16384): the warps a row has in flight
@@ -546,8 +548,8 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
         const size_t smem = ACT_ONLY ? 0 : (size_t)warps * 2 * kTilePairs * sizeof(f2);
 #define TPB_PREP_CASE(UU)                                                                               \
     case UU: {                                                                                          \
-        auto kern = ACT_ONLY && P.ahead == 0 ? convrot_prep_kernel<T, UU, OP, ACT_ONLY, false, !ACT_ONLY>   \
-                                             : convrot_prep_kernel<T, UU, OP, ACT_ONLY, false>;         \
+        auto kern = kRms && P.ahead == 0 ? convrot_prep_kernel<T, UU, OP, ACT_ONLY, false, !kRms>       \
+                                         : convrot_prep_kernel<T, UU, OP, ACT_ONLY, false>;             \
         static tpb_per_device_once smem_set;                                                            \
         if (smem > 48 * 1024) err = tpb_set_max_smem_once(h, kern, (int)kMaxPrepSmem, smem_set);        \
         if (err == cudaSuccess) err = tpb_launch_pdl(kern, grid, block, smem, st, P);                   \

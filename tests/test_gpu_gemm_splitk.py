@@ -6,6 +6,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
+from graph_nodes import kernels  # noqa: E402
 from oracle import oracle  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -53,40 +54,9 @@ def test_split_is_exact(be, m, n, k):
 # -- every width and cluster size, and which one a call takes ------------------------------------
 
 
-def _kernels(fn):
-    """(name, CTAs) of every kernel that fn launches, from the nodes of a captured graph."""
-    import ctypes as C
-
-    class Params(C.Structure):
-        _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("shared", C.c_uint), ("params", C.c_void_p),
-                    ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
-
-    cu = C.CDLL("libcuda.so.1")
-    stream = torch.cuda.Stream()
-    with torch.cuda.stream(stream):
-        g = torch.cuda.CUDAGraph(keep_graph=True)
-        with torch.cuda.graph(g, stream=stream):
-            fn()
-        n = C.c_size_t(0)
-        raw = C.c_void_p(g.raw_cuda_graph())
-        assert cu.cuGraphGetNodes(raw, None, C.byref(n)) == 0
-        nodes = (C.c_void_p * n.value)()
-        assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
-        out = []
-        for node in nodes:
-            p, name = Params(), C.c_char_p()
-            if cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) != 0:
-                continue
-            get, arg = (cu.cuFuncGetName, p.func) if p.func else (cu.cuKernelGetName, p.kern)
-            assert get(C.byref(name), C.c_void_p(arg)) == 0
-            out.append((name.value.decode(), p.grid[0]))
-    torch.cuda.synchronize()
-    return out
-
-
 def _split_of(be, y, wd, wsd, n):
     """(columns, parts) of the GEMM that be._gemm launches for y; None: K in one chain."""
-    (name, ctas), = _kernels(lambda: be._gemm(y, wd, wsd, n, 8))
+    (name, ctas, *_), = kernels(lambda: be._gemm(y, wd, wsd, n, 8))
     if "splitk" not in name:
         return None
     bn = next(b for b in (64, 128, 192) if f"splitk_kernelILi{b}E" in name)
