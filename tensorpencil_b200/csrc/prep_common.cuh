@@ -235,8 +235,10 @@ __device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
 // AHEAD: the kernel can ask rows into L2 (P.ahead).  RMS norm over few rows, which asks for none, has a variant without: alone 18 x 11008 bf16
 // 4.5 -> 4.3 us, 77 x 9216 f32 6.1 -> 5.8; in front of the quantiser with f32 inputs it takes 64 registers a thread instead of 72, so that an eighth
 // CTA of four warps fits an SM (1170 x 3328 11.3 -> 10.1 us).
+// The gated rows of 33 to 48 units need two CTAs an SM and so at most 128 registers a thread (with 132: 2290 x 18944 f32 SiLU 173 -> 305 us, 689 x 22272
+// bf16 sigmoid 54 -> 77).
 template <typename T, int UPW, int OP, bool ACT_ONLY, bool ONE_WARP, bool AHEAD = true>
-__global__ void __launch_bounds__((UPW == 1 ? kMaxWarpsWide : kMaxWarps) * 32)
+__global__ void __launch_bounds__((UPW == 1 ? kMaxWarpsWide : kMaxWarps) * 32, UPW == 3 && (OP == OP_SILU_MUL || OP == OP_SIGMOID_MUL) ? 2 : 0)
 convrot_prep_kernel(const PrepParams P) {
     __shared__ float s_max[kMaxWarpsWide];
     __shared__ int s_sum[kMaxWarpsWide];

@@ -29,3 +29,11 @@ def test_rms_norm_of_f32_rows(be, m, k, rows):
     x = torch.ones((m, k), device="cuda")
     mod = torch.ones(2 * k, device="cuda")
     assert _only(lambda: be.prepRmsMod(x, mod, m, k, 0, k, 1e-6)).ctas_per_sm >= rows
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("k", [16640, 18944, 22016, 24576])
+def test_gated_rows_of_many_columns(be, k, dtype):
+    a = torch.ones((3, k), device="cuda", dtype=dtype)
+    assert _only(lambda: be.prepSiluMul(a, a, 3, k)).ctas_per_sm >= 2
+    assert _only(lambda: be.prepSigmoidMul(a, a, 3, k, 4)).ctas_per_sm >= 2
