@@ -265,7 +265,7 @@ int tpb_convrot_gemm_group(tpb_handle_t h, tpb_stream_t stream, int count, void 
     }
     TPB_CHECK_ARG(h, m >= 0 && m < (1ll << 31), "gemm_group: bad m");
     if (m == 0) return TPB_OK;
-    return tpb_launch_gemm_group(h, (cudaStream_t)stream, count, y, y_dtype, ldy, q, act_scale, w, w_scale, w_bits, m, n, k);
+    return tpb_launch_gemm_group(h, (cudaStream_t)stream, count, y, y_dtype, ldy, q, act_scale, act_sum, w, w_scale, w_bits, m, n, k);
 }
 
 int tpb_q8_1_quantize(tpb_handle_t h, tpb_stream_t stream, const float *x, int64_t n_elems,

@@ -453,8 +453,8 @@ int tpb_launch_gemm_silu_pair(tpb_handle_t h, cudaStream_t st, void *y, int y_dt
 // the one-CTA kernel fits a single weight so much better that it pays: two weights of m 2048, n 12288, k 512 to bf16 46 us one by one,
 // 54 together, of m 256, n 3072, k 256 7.3 / 8.0; but four of m 256, n = k = 3072 41 / 17, four of m 1111, n 3072, k 12288 143 / 141.
 int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *const *y, int y_dtype, int64_t ldy,
-                          const int8_t *q, const float *act_scale, const void *const *w, const float *const *w_scale,
-                          int w_bits, int64_t m, int64_t n, int64_t k) {
+                          const int8_t *q, const float *act_scale, const int32_t *act_sum, const void *const *w,
+                          const float *const *w_scale, int w_bits, int64_t m, int64_t n, int64_t k) {
     const Epilogue epi = y_dtype == TPB_BF16 ? EPI_BF16 : EPI_F32;
     double one_us = 0.0;
     pick_tile(h, epi, m, n, k, &one_us);
@@ -471,7 +471,7 @@ int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *cons
     const double together_us = (small ? 1.0 : 0.96) * tile_us(h->sm_count, P256, epi, m, n, k, count);
     if (h->opt_gemm_one_cta || scratch_for_one || together_us > count * one_us) {
         for (int g = 0; g < count; g++) {
-            const int rc = tpb_launch_gemm(h, st, y[g], y_dtype, ldy, q, act_scale, nullptr, w[g], w_bits, w_scale[g], m, n, k,
+            const int rc = tpb_launch_gemm(h, st, y[g], y_dtype, ldy, q, act_scale, act_sum, w[g], w_bits, w_scale[g], m, n, k,
                                            nullptr, 0, nullptr, nullptr);
             if (rc != TPB_OK) return rc;
         }

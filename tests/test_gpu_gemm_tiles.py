@@ -173,3 +173,26 @@ def test_large_int4_group_needs_scratch_for_all_weights_on_both_routes(n):
     b.gemmGroup(ys, ws, sc, n, 4)
     b.status_poll()
     b.close()
+
+
+def test_int4_group_one_by_one_with_the_kernel_that_unpacks(monkeypatch):
+    """One by one, each weight of a group takes the route of a single call, also the one that unpacks int4 inside the GEMM and corrects its
+    unsigned products by the activations' sums."""
+    from tensorpencil_b200.backend import Backend
+    monkeypatch.setenv("TPB_W4_FUSED", "1")
+    b = Backend(0)
+    m, n, k = 2048, 12288, 512
+    g = torch.Generator(device="cuda").manual_seed(5)
+    b.reserveW4(2 * n, k)
+    b._prep(torch.randn((m, k), device="cuda", generator=g), m, k, 4)
+    ws = [torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=g) for _ in range(2)]
+    sc = [torch.rand(n, device="cuda", generator=g) + 0.5 for _ in ws]
+    want = [torch.empty((m, n), dtype=torch.bfloat16, device="cuda") for _ in ws]
+    for y, w, s in zip(want, ws, sc):
+        b._gemm(y, w, s, n, 4)
+    got = [torch.full((m, n), 3.0, dtype=torch.bfloat16, device="cuda") for _ in ws]
+    b.gemmGroup(got, ws, sc, n, 4)
+    b.status_poll()
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
+    assert _kernels_in(lambda: b.gemmGroup(got, ws, sc, n, 4)) == 2        # nothing is widened
+    b.close()
