@@ -293,7 +293,7 @@ Tile pick_tile(tpb_handle_t h, Epilogue epi, int64_t m, int64_t n, int64_t k, do
 // chain / split: m 16, n 1024, k 12288 29.4 / 8.3; m 64, n 3072, k 6144 16.8 / 8.8; m 256, n 1024, k 3072 10.1 / 6.3; m 256, n = k = 3072 10.5 / 9.0;
 // m 297, n 3072, k 12288 30.6 / 22.2.  Over 384 shapes and epilogues with m 16 .. 1111 the choice is 1.28 x as fast as
 // one chain on average and nowhere more than 2 % slower.  Several rounds of clusters lost everywhere (m 512, n 5008, k 3072: 13.9 / 25 and more).
-struct Split { int bn = 0, parts = 1; };
+struct Split { int bn = 0, parts = 1; double us = 0.0; };
 Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta_us) {
     static const struct { int bn; double fixed, per_block, rows, rows_part, load; } kCost[] = {
         {64, 2.84, 0.260, 1.51, -2.13, 0.112}, {128, 3.10, 0.345, 2.08, -2.10, 0.080}, {192, 3.49, 0.352, 2.85, -1.90, 0.265}};
@@ -306,6 +306,7 @@ Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta
         if (h->opt_gemm_split_parts <= blocks && tiles <= h->max_clusters[h->opt_gemm_split_parts]) {
             best.bn = h->opt_gemm_split_bn;
             best.parts = h->opt_gemm_split_parts;
+            best.us = t_best;
         }
         return best;
     }
@@ -319,7 +320,7 @@ Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta
             if (us < t_best) {
                 best.bn = c.bn;
                 best.parts = parts;
-                t_best = us;
+                best.us = t_best = us;
             }
         }
     }
@@ -452,12 +453,16 @@ int tpb_launch_gemm_silu_pair(tpb_handle_t h, cudaStream_t st, void *y, int y_dt
 // and drains once instead of once per weight, and the last round is shared by all of them.  One by one where a tile of
 // the one-CTA kernel fits a single weight so much better that it pays: two weights of m 2048, n 12288, k 512 to bf16 46 us one by one,
 // 54 together, of m 256, n 3072, k 256 7.3 / 8.0; but four of m 256, n = k = 3072 41 / 17, four of m 1111, n 3072, k 12288 143 / 141.
+// A weight whose K is split over a cluster is a shorter single call, but a split launch right behind another takes up to a fifth more than alone, so
+// it has to be 15 % better than the group: us, together / one by one with K split: two of m 49, n 384, k 8960 27.3 / 11.8, three of m 2, n 704, k 7936 25.8 /
+// 17.1; but four of m 3, n 960, k 4608 18.1 / 23.9.  Over 114 groups of m 1 .. 700 the choice is 0.5 % off the better route on average (8.8 without).
 int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *const *y, int y_dtype, int64_t ldy,
                           const int8_t *q, const float *act_scale, const int32_t *act_sum, const void *const *w,
                           const float *const *w_scale, int w_bits, int64_t m, int64_t n, int64_t k) {
     const Epilogue epi = y_dtype == TPB_BF16 ? EPI_BF16 : EPI_F32;
     double one_us = 0.0;
     pick_tile(h, epi, m, n, k, &one_us);
+    const Split split = pick_split(h, m, n, k, one_us);
     // A reservation that covers one int4 weight only is enough for small problems, as it was when they always ran one by one.
     const bool small = (m + 255) / 256 * ((n + 255) / 256) < h->sm_count / 2;
     const bool scratch_for_one = w_bits == 4 && small && h->w4_scratch_bytes < (size_t)count * (size_t)n * (size_t)k;
@@ -469,7 +474,7 @@ int tpb_launch_gemm_group(tpb_handle_t h, cudaStream_t st, int count, void *cons
     }
     // the pair's bonus where it holds (pick_tile): in a launch long enough to meet the power cap
     const double together_us = (small ? 1.0 : 0.96) * tile_us(h->sm_count, P256, epi, m, n, k, count);
-    if (h->opt_gemm_one_cta || scratch_for_one || together_us > count * one_us) {
+    if (h->opt_gemm_one_cta || scratch_for_one || together_us > count * one_us || (split.parts > 1 && 0.85 * together_us > count * split.us)) {
         for (int g = 0; g < count; g++) {
             const int rc = tpb_launch_gemm(h, st, y[g], y_dtype, ldy, q, act_scale, act_sum, w[g], w_bits, w_scale[g], m, n, k,
                                            nullptr, 0, nullptr, nullptr);

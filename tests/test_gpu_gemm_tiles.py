@@ -196,3 +196,11 @@ def test_int4_group_one_by_one_with_the_kernel_that_unpacks(monkeypatch):
     assert all(torch.equal(x, y) for x, y in zip(got, want))
     assert _kernels_in(lambda: b.gemmGroup(got, ws, sc, n, 4)) == 2        # nothing is widened
     b.close()
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("count,m,n,k,together", [(2, 49, 384, 8960, False), (3, 2, 704, 7936, False), (2, 21, 384, 5888, False), (4, 3, 960, 4608, True),
+                                                  (3, 7, 2192, 3328, True)])
+def test_group_route_knows_the_split(be, bits, count, m, n, k, together):
+    """Few weights whose single calls split K over a cluster go one by one; more of them together all the same."""
+    test_group_route_and_results(be, bits, count, m, n, k, together)
