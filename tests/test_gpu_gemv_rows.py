@@ -57,3 +57,8 @@ def test_rows_do_not_depend_on_their_neighbours(be, fmt, m, n, k):
     be.status_poll()
     assert bool(torch.isfinite(got).all())
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n,k", [(2 * SMS * 16 - 1, 2048), (2 * SMS * 20, 2048), (2 * SMS * 20 + 1, 2304), (2 * SMS * 24 + 1, 2048), (2600, 4096), (5119, 5120), (9999, 2048)])
+def test_rows_do_not_depend_on_their_neighbours_at_two_activation_rows(be, n, k):
+    test_rows_do_not_depend_on_their_neighbours(be, "q8_0", 2, n, k)

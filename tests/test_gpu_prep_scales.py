@@ -1,6 +1,7 @@
 """The activation prep's scale and rounding where its fast paths end: the quotient absmax / maxq over the whole range of magnitudes, rows whose
-absmax is infinite, values at and beside half-integer quotients, and rows behind and ahead of those that ask the next ones into L2.
-Scales and quants are the oracle's bits."""
+absmax is infinite, values at and beside half-integer quotients, and launches of many waves, whose rows ask later ones into L2 where
+inputs have 16 bits or pass through RMS norm.  Scales and quants are the oracle's bits, or those of the same rows in short launches, which ask for
+none."""
 import numpy as np
 import pytest
 
@@ -77,3 +78,36 @@ def test_more_rows_than_are_resident(be, m, k):
     q, s, _ = run(be, x, 8)
     assert np.array_equal(s[pick].view(np.uint32), s_ref.view(np.uint32))
     assert np.array_equal(q[pick], q_ref)
+
+
+@pytest.mark.parametrize("op,dtype", [("plain", torch.bfloat16), ("plain", torch.float16), ("silu", torch.bfloat16), ("sigmoid", torch.bfloat16),
+                                      ("rms", torch.bfloat16), ("rms", torch.float32), ("rms alone", torch.bfloat16)])
+@pytest.mark.parametrize("m,k", [(23701, 512), (7411, 3072), (1531, 12288), (3709, 12288)])
+def test_rows_of_long_launches_are_those_of_short_ones(be, op, dtype, m, k):
+    """More than five waves on 148 SMs and not a whole number of them, so that the requests end inside the last one (RMS norm has fewer warps a row
+    and reaches five waves of 12288 columns at 3700 rows)."""
+    if op.startswith("rms") and m == 1531:
+        pytest.skip("fewer than five waves")
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn((m, k), device="cuda", generator=g).to(dtype)
+    y = torch.randn((m, k), device="cuda", generator=g).to(dtype) if op in ("silu", "sigmoid") else None
+    mod = torch.randn(2 * k, device="cuda", generator=g)
+
+    def rows(a, b):
+        n = b - a
+        if op == "rms alone":
+            out = torch.empty((n, k), device="cuda")
+            be.rmsMod(x[a:b], out, mod, n, k, 0, k, 1e-6)
+            return (out,)
+        if op == "plain":
+            be._prep(x[a:b], n, k, 8)
+        elif op == "rms":
+            be.prepRmsMod(x[a:b], mod, n, k, 0, k, 1e-6)
+        else:
+            (be.prepSiluMul if op == "silu" else be.prepSigmoidMul)(x[a:b], y[a:b], n, k)
+        return be.i8_x[: n * k].clone().view(n, k), be.i8_scale[:n].clone(), be.i8_sum[:n].clone()
+
+    got = rows(0, m)
+    want = [torch.cat(parts) for parts in zip(*[rows(a, min(a + 500, m)) for a in range(0, m, 500)])]
+    be.status_poll()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
