@@ -535,13 +535,13 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
     } else {
         // One unit per half-warp, up to 16 warps a row, where the row fits that way (k <= 16384): the warps a row has in flight
         // hide its latencies, and with two units each they are half as many.  us, 8 warps of two units / one unit each: SiLU gate 4608 x 12288 bf16
-        // 152 / 82, plain f32 1111 x 8448 13.4 / 12.9, 4608 x 13312 78.9 / 74.0, bf16 512 x 12288 11.3 / 10.1, 4608 x 12288 58.1 / 57.9.
-        // The plain prep of many rows keeps two units where as many rows fit an SM without a half-warp of them idle: at 19 and 20 units (four rows
-        // of five warps against three of ten; f32 4608 x 10240 48.9 / 52.1) and from 31 on (4608 x 16128 86.5 / 88.3).  So does RMS norm,
-        // whose sum of squares has always been taken in that order.
+        // 152 / 82, plain f32 1111 x 8704 15.0 / 13.9, 4608 x 13312 75.8 / 67.7, 4608 x 16384 82.5 / 79.8, bf16 4608 x 12288 51.7 / 50.2.
+        // The plain prep of many rows keeps two units where more rows fit an SM that way: at 19 and 20 units (four rows of five warps against three of
+        // ten: 4608 x 10240 f32 47.3 / 48.7, bf16 42.8 / 43.2, though 1111 rows 16.0 / 14.9 and 13.6 / 13.3).  So does RMS norm, whose sum of squares has
+        // always been taken in that order.
         constexpr bool kGated = OP == OP_SILU_MUL || OP == OP_SIGMOID_MUL;
         const bool wide = n_units <= 2 * kMaxWarpsWide &&
-                          (kGated || (OP == OP_PLAIN && (m <= h->sm_count || !(n_units == 19 || n_units == 20 || n_units > 30))));
+                          (kGated || (OP == OP_PLAIN && (m <= h->sm_count || !(n_units == 19 || n_units == 20))));
         const int max_warps = wide ? kMaxWarpsWide : kMaxWarps;
         const int upw = (n_units + 2 * max_warps - 1) / (2 * max_warps);  // 1..4 for k <= 32768
         const int warps = (n_units + 2 * upw - 1) / (2 * upw);

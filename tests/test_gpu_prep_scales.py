@@ -111,3 +111,9 @@ def test_rows_of_long_launches_are_those_of_short_ones(be, op, dtype, m, k):
     want = [torch.cat(parts) for parts in zip(*[rows(a, min(a + 500, m)) for a in range(0, m, 500)])]
     be.status_poll()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("k", [9728, 10240, 15360, 15872, 16384])
+def test_one_and_two_units_a_half_warp(be, k):
+    """Both sides of the rule at more rows than SMs."""
+    check(be, np.random.default_rng(k).standard_normal((160, k)).astype(np.float32), 8)
