@@ -292,7 +292,7 @@ Tile pick_tile(tpb_handle_t h, Epilogue epi, int64_t m, int64_t n, int64_t k, do
 // parts are sent and added, and the bytes that all SMs load (us, fitted to 128 shapes x 18 choices, rms error 6-8 %).  us, one
 // chain / split: m 16, n 1024, k 12288 29.4 / 8.3; m 64, n 3072, k 6144 16.8 / 8.8; m 256, n 1024, k 3072 10.1 / 6.3; m 256, n = k = 3072 10.5 / 9.0;
 // m 297, n 3072, k 12288 30.6 / 22.2.  Over 384 shapes and epilogues with m 16 .. 1111 the choice is 1.28 x as fast as
-// one chain on average and nowhere more than 2 % slower.  Several rounds of clusters lost everywhere (m 512, n 5008, k 3072: 13.9 / 25 and more).
+// one chain on average and 2 % slower at worst, over 200 others with m 1 .. 1400 4 % at worst (m 642, n 1424, k 512 gated 6.8 / 7.1).  Several rounds of clusters lost everywhere (m 512, n 5008, k 3072: 13.9 / 25 and more).
 struct Split { int bn = 0, parts = 1; double us = 0.0; };
 Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta_us) {
     static const struct { int bn; double fixed, per_block, rows, rows_part, load; } kCost[] = {

@@ -615,15 +615,16 @@ int tpb_launch_q8_0_gemv_q8n(tpb_handle_t h, cudaStream_t st, float *y, const vo
                              int64_t rows, int64_t cols, const void *xq, int ng, int row_off,
                              int n_total) {
     // Two kernels.  The dp4a streaming kernel below costs one dp4a per weight word and activation row: the fastest
-    // for one row, 2-10 % slower with each further row, and much slower once its activations crowd the rings out of
+    // for one row, 2-5 % slower with the second and 6-20 % with each further one, and much slower once its activations crowd the rings out of
     // shared memory.  The kernel that keeps the activations in registers and takes the block sums from mma.sync
-    // (qgemv_mma.cu) costs the same whatever M is, but 0-4 us more than the dp4a kernel's single row (more where its
+    // (qgemv_mma.cu) costs the same whatever M is, but 2-7 us more than the dp4a kernel's single row (more where its
     // per-warp K slices are padded, K = 4096: 4 block pairs in MMAs built for 6, and where it needs two passes
-    // over K).  Measured on ten decode shapes, M = 1 .. 8 (us, dp4a / mma): 17408 x 5120  17.6 19.1 21.0 23.8 /
-    // 19.2-20.0;  5120 x 17408  21.1 22.9 25.4 / 19.9-21.4 (few long rows: 2.9 of
-    // them a warp for two-row stages; eighteen warps with one step each take 17.8 and 18.8 for one and two activation rows);  32000 x 4096  22.6 22.7 24.8 26.7 29.9 / 27.1-28.7;  4096 x 14336  11.6 12.7 13.7 15.1
-    // 16.9 26.7 / 15.3-16.2;  8192 x 28672  41.0 42.2 69.6 / 49.8-53.0;  28672 x 8192  41.4 42.4 43.6 47.9 /
-    // 41.4-44.9.  The rule below follows that table.  TPB_GEMV_KERNEL=dp4a / mma forces one.
+    // over K).  Measured on ten decode shapes, M = 1 .. 8 (us, dp4a / mma): 17408 x 5120  16.5 17.0 20.9 23.7 /
+    // 19.5-20.2;  5120 x 17408  17.0 17.9 25.3 / 20.1-21.4;  32000 x 4096  22.2 22.5 24.6 26.6 29.8 / 27.9-29.0;  4096 x 14336  11.2 11.9
+    // 13.2 14.5 16.3 26.2 / 15.2-16.2;  14336 x 4096  11.3 11.6 14.4 16.4 / 15.7-16.5;  8192 x 8192  12.6 13.4 14.9 16.6 / 16.0-16.6;  8192 x 28672
+    // 41.1 42.9 64.1 / 48.1-52.9;  28672 x 8192  39.2 40.2 42.1 47.6 / 41.3-43.3;  6144 x 4096  6.4 6.9 8.2 9.4 / 10.0-10.6;  4096 x 11008  10.0 10.6 11.6
+    // 13.2 14.5 / 14.3-15.5.  The rule below is 0.4 % off the better one on average over these 70 calls (at worst 9 %, 4096 x 14336 at M = 4), 0.1 % over 50
+    // others at M = 1 and 2.  TPB_GEMV_KERNEL=dp4a / mma forces one.
     GemvPlan plan;
     bool planned = false;
     {

@@ -936,8 +936,8 @@ int launch_q6k_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
         const size_t act_r = (size_t)M * (p.cols / 64) * kActPairBytes + (size_t)M * p.nblk * 4 + (size_t)M * (p.cols / 16) * 4;
         const size_t limit_r = (size_t)h->smem_optin - 1024;
         const int s_r = act_r + 256 < limit_r ? (int)((limit_r - act_r - 256) / ((size_t)kRingRows * kQ6RowStage + 16)) : 0;
-        // measured (us, per-warp rings / ring): K = 17408 -> N = 5120 28.9 / 23.5, 32000 x 4096 34.1 / 27.7, but
-        // 17408 x 5120 22.2 / 27.8 and 8192 x 8192 14.9 / 15.6 at M = 1; at M = 2 4096 x 14336 19.4 / 15.9
+        // measured (us, per-warp rings / ring): 5120 x 17408 23.7 / 23.3, 17408 x 5120 22.0 / 27.5 and 8192 x 8192 14.8 / 15.2 at M = 1; at M = 2 4096 x
+        // 14336 19.4 / 15.7, 8192 x 8192 16.9 / 16.5.  The many rows were drawn with ranges cut at any row (32000 x 4096 34.1 / 27.7); in pairs 23.9 / 27.3
         const bool many_rows = p.rows > 10 * 16 * h->sm_count;
         const bool pick = many_rows || p.cols >= (M == 1 ? 16384 : 8192);
         if (s_r >= 3 && (force == 1 || (force == 0 && pick))) return launch_q6k_ring<M>(h, st, p, s_r > 12 ? 12 : s_r, act_r);
@@ -1038,10 +1038,11 @@ int launch_fmt_m(tpb_handle_t h, cudaStream_t st, const KGemvParams &p) {
     const int n_units = p.cols / 64;
     bool u3 = false;
     if constexpr (M <= 4) u3 = kq_three_units(M, p.cols);
-    // The ring kernel for one or two activation rows where the per-warp rings serialise: rows of several chunks
-    // (K = 17408, M = 1: q4_k 21.5 -> 14.4 us, q4_0 18.2 -> 12.7, q5_k 25.1 -> 18.2) and many rows per warp
-    // (32000 x 4096: q4_k 28.9 -> 19.2 us).  With short rows and few of them per warp the two are within 5 %
-    // either way, and from four activation rows on the dot products set the time in both.
+    // The ring kernel for one or two activation rows where per-warp rings serialise: rows of several chunks (us at M = 1, per-warp rings / ring: 5120 x
+    // 17408 q4_k 14.6 / 12.9, q4_0 14.2 / 12.5, q5_k 17.6 / 15.3, iq4_nl 25.5 / 22.2) and many rows per warp.  The line was drawn with ranges of
+    // rows cut at any row; in pairs the per-warp rings are the faster for many rows, but for iq4_nl (32000 x 4096 q4_k 16.0 / 18.1, 21095 x 8192 20.7 /
+    // 24.2, iq4_nl 38.7 / 36.6), and as before the ring for few rows of one chunk (2191 x 5632 q5_k 6.2 / 3.9).  Over 160 calls at M = 1 and 2
+    // the choice is 5 % off the better kernel on average.  From four activation rows on the dot products set the time in both.
     if constexpr (M <= 2) {
         const int force = k_kernel_override();
         const int cpr = (n_units + (u3 ? 96 : 64) - 1) / (u3 ? 96 : 64);
