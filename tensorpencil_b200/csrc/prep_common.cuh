@@ -520,9 +520,12 @@ int launch_prep_op(tpb_handle_t h, cudaStream_t st, const PrepParams &P0, int64_
     // from five waves on; f32 rows are long enough in flight, two of them more so, and a short launch only gets a second stream beside its first.
     // us without / a wave ahead / half of one: bf16 4608 x 12288 plain 50.8 / 49.9 / 49.5, SiLU gate 85.7 / 75.9 / 74.6, RMS 99.8 / 95.0 / 93.5; f32
     // RMS 4608 x 12288 110.7 / 105.1 / 102.3; but f32 plain 4608 x 3072 16.3 / 18.8 / 17.3, SiLU gate 113 / 121 / 118, bf16 1111 x 12288 plain 15.0 / 15.3 / 15.1.
+    // None for stand-alone RMS norm of f32 rows above 80 KB, which also writes as much as it reads (without / half a wave: 5967 x 18688 199 / 179, but
+    // 5827 x 20992 220 / 236, 4257 x 24064 182 / 235, 4595 x 26112 339 / 380).
+    const bool asks = sizeof(T) == 2 || (OP == OP_RMS_MOD && !(ACT_ONLY && k > 20480));
     auto set_ahead = [&](int rows_per_sm) {
         const int64_t wave = (int64_t)rows_per_sm * h->sm_count;
-        P.ahead = (sizeof(T) == 2 || OP == OP_RMS_MOD) && m >= 5 * wave ? (int)(wave / 2) : 0;
+        P.ahead = asks && m >= 5 * wave ? (int)(wave / 2) : 0;
     };
     constexpr bool kRms = OP == OP_RMS_MOD;
     cudaError_t err = cudaSuccess;
