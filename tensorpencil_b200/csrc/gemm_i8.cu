@@ -292,7 +292,7 @@ Tile pick_tile(tpb_handle_t h, Epilogue epi, int64_t m, int64_t n, int64_t k, do
 // parts are sent and added, and the bytes that all SMs load (us, fitted to 128 shapes x 18 choices, rms error 6-8 %).  us, one
 // chain / split: m 16, n 1024, k 12288 29.4 / 8.3; m 64, n 3072, k 6144 16.8 / 8.8; m 256, n 1024, k 3072 10.1 / 6.3; m 256, n = k = 3072 10.5 / 9.0;
 // m 297, n 3072, k 12288 30.6 / 22.2.  Over 384 shapes and epilogues with m 16 .. 1111 the choice is 1.28 x as fast as
-// one chain on average and 2 % slower at worst, over 200 others with m 1 .. 1400 4 % at worst (m 642, n 1424, k 512 gated 6.8 / 7.1).  Several rounds of clusters lost everywhere (m 512, n 5008, k 3072: 13.9 / 25 and more).
+// one chain on average and 2 % slower at worst, over 200 others with m 1 .. 1400 4 % at worst (m 642, n 1424, k 512 gated 6.8 / 7.1), at k 256 5 % (m 204, n 912 to s32 3.1 / 3.3).  Several rounds of clusters lost everywhere (m 512, n 5008, k 3072: 13.9 / 25 and more).
 struct Split { int bn = 0, parts = 1; double us = 0.0; };
 Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta_us) {
     static const struct { int bn; double fixed, per_block, rows, rows_part, load; } kCost[] = {
@@ -311,6 +311,9 @@ Split pick_split(tpb_handle_t h, int64_t m, int64_t n, int64_t k, double one_cta
         return best;
     }
     const double rows = (double)(m < BM ? m : BM) / BM;
+    // Parts of a single K block of full tiles with few columns: there is next to no chain, and the one-chain kernel's epilogue stores less than its cost
+    // says (m 193, n 32, k 256 3.0 one chain / 3.35 split; but m 5, n 16 2.8 / 2.3, m 185, n 1360 gated 4.9 / 3.85).
+    if (blocks < 4 && m > BM && n <= 96) return best;
     for (const auto &c : kCost) {
         const int64_t tiles = (m + BM - 1) / BM * ((n + c.bn - 1) / c.bn);
         for (int parts = 2; parts <= kMaxSplit && parts <= blocks; parts++) {

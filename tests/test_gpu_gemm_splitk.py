@@ -138,3 +138,10 @@ def test_one_chain_is_kept_where_asked_for(monkeypatch, env, m, n, k):
     assert _split_of(b, torch.empty((m, n), device="cuda"), wd, wsd, n) is None
     _check(b, m, n, k, wd, wsd, want)
     b.close()
+
+
+@pytest.mark.parametrize("m,n,k,split", [(193, 32, 256, False), (319, 16, 256, False), (5, 16, 256, True), (128, 96, 256, True), (193, 32, 512, True)])
+def test_the_rule_leaves_short_chains_of_few_columns(be, m, n, k, split):
+    wd, wsd, want = _problem(be, m, n, k)
+    assert (_split_of(be, torch.empty((m, n), device="cuda"), wd, wsd, n) is not None) == split
+    _check(be, m, n, k, wd, wsd, want)
